@@ -302,8 +302,12 @@ rt_status ensure_scratch(rt_ctx* ctx, long long n_rays, int levels, long long n_
     take(&ctx->d_bar, 2);
     if (pass == 0) CK(dalloc(ctx->scratch, &block, used));
   }
-  CK(cudaMemcpy(ctx->d_levels, ctx->h_levels.data(), (Lv + 1) * sizeof(LevelBuf), cudaMemcpyHostToDevice));
-  CK(cudaMemset(ctx->d_bar, 0, 2 * sizeof(unsigned)));
+  // on the stream of the kernels that read them: it does not wait for the
+  // legacy stream, and a clear queued there behind another thread's work
+  // could land in a running k_levels' arrival count
+  CK(cudaMemcpyAsync(ctx->d_levels, ctx->h_levels.data(), (Lv + 1) * sizeof(LevelBuf), cudaMemcpyHostToDevice,
+                     ctx->stream));
+  CK(cudaMemsetAsync(ctx->d_bar, 0, 2 * sizeof(unsigned), ctx->stream));
   ctx->d_counts = ctx->d_res->counts;
   ctx->d_nhits = ctx->d_res->nhits;
   ctx->d_stats = ctx->d_res->stats;
