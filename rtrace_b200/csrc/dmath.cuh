@@ -263,6 +263,18 @@ struct StdRng {
   }
 };
 
+// A walk's reference to a BVH child: the node's index, or for a leaf of 1 to
+// RTB_LEAF primitives, below zero, the first one's position and the count.
+// 32 bits hold positions below RTB_MAX_PRIMS.  A mesh that large would take
+// 280 bytes a triangle on the device, 150 GB, and 184 more while it is
+// prepared: uploads refuse more triangles than that.
+#define RTB_LEAF 4
+#define RTB_MAX_PRIMS (1 << 29)
+#define RTB_WALK_DONE 0x7fffffff
+RTB_HD int walk_ref(int idx, int cnt) { return cnt ? ~(idx << 2 | (cnt - 1)) : idx; }
+RTB_HD int leaf_first(int ref) { return ~ref >> 2; }
+RTB_HD int leaf_count(int ref) { return (~ref & 3) + 1; }
+
 // The primary ray that place i of level 0's walk order takes: 32 consecutive
 // places are a tile of TW x TH pixels with all their samples (8 x 4, 4 x 4,
 // 4 x 2, 2 x 2 for 1, 2, 4, 8 samples), not a run of one row.

@@ -593,16 +593,14 @@ __device__ __forceinline__ bool box_hit_f(const float* mn, const float* mx, cons
   return f.all || (tl <= th && th >= 0.0f && !(tl > tmax));
 }
 
-// BVH walks by one thread each: a reference to a child is its node index,
-// or for a leaf ~(first << 4 | count).  A walk descends until it meets a
-// leaf or runs out of nodes and only then tests the leaf, so that the lanes
-// of a warp run the (double) leaf tests together rather than one lane's
-// leaf at a time between the others' (single-precision) node steps.  (Warp
-// packets, one shared walk for the 16 rays of a light, cost 2.5 ms where
-// this costs 1.4 on the rays the icosphere frame's cones leave: those cones
-// are wide, and their rays meet different leaves.)
-#define RTB_WALK_DONE 0x7fffffff
-__device__ __forceinline__ int walk_ref(int idx, int cnt) { return cnt ? ~(idx << 4 | cnt) : idx; }
+// BVH walks by one thread each, over references to children (walk_ref).  A
+// walk descends until it meets a leaf or runs out of nodes and only then
+// tests the leaf, so that the lanes of a warp run the (double) leaf tests
+// together rather than one lane's leaf at a time between the others'
+// (single-precision) node steps.  (Warp packets, one shared walk for the 16
+// rays of a light, cost 2.5 ms where this costs 1.4 on the rays the icosphere
+// frame's cones leave: those cones are wide, and their rays meet different
+// leaves.)
 
 // The pruning bound t * RTB_PRUNE_REL + RTB_PRUNE_ABS, rounded up.
 __device__ __forceinline__ float prune_bound(double t) {
@@ -647,7 +645,7 @@ __device__ __forceinline__ void closest_bvh(const float4* fbvh, V3 o, V3 d, doub
       }
     }
     if (cur == RTB_WALK_DONE) return;
-    const int first = ~cur >> 4, cnt = ~cur & 15;
+    const int first = leaf_first(cur), cnt = leaf_count(cur);
     double t = 0.0;
     for (int j = first; j < first + cnt; j++) t = test(j);
     bound = prune_bound(t);
@@ -1052,7 +1050,7 @@ __device__ __forceinline__ int shaft_collect(const DScene& S, const Cone& k, int
         }
       }
       if (cur == RTB_WALK_DONE) break;
-      const int first = ~cur >> 4, cnt = ~cur & 15;
+      const int first = leaf_first(cur), cnt = leaf_count(cur);
       for (int j = first; j < first + cnt; j++) {
         int at = j;
         if (mesh) {
@@ -1123,7 +1121,7 @@ __device__ __forceinline__ bool shadow_bvh(const float4* fbvh, V3 o, V3 d, doubl
       }
     }
     if (cur == RTB_WALK_DONE) return false;
-    const int first = ~cur >> 4, cnt = ~cur & 15;
+    const int first = leaf_first(cur), cnt = leaf_count(cur);
     for (int j = first; j < first + cnt; j++)
       if (test(j)) return true;
     cur = sp ? stack[--sp] : RTB_WALK_DONE;

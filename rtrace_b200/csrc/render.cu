@@ -789,7 +789,7 @@ void parallel_ranges(long long n, F f) {
 // Triangles per mesh BVH leaf.  With single-precision box tests 4 is
 // fastest on the 82k-triangle mesh frame (7.21 ms; 2: 7.31, 3: 7.26,
 // 5: 7.28, 6: 7.30, 8: 7.39, 12: 7.68); with double boxes it was 8.
-const int kMeshLeaf = 4;
+const int kMeshLeaf = RTB_LEAF;
 // Meshes from this many triangles up are prepared on the device (median
 // split BVH, tens of ms for millions of triangles); smaller ones on the
 // host with a binned SAH BVH (about 7% fewer node visits per ray, 4% on the
@@ -807,8 +807,8 @@ std::string prep_mesh_kd(const rt_mesh_desc& md, MeshPrep* P) {
   }
   long long nt = md.n_triangles;
   if (nt < 0 || md.n_nodes < 0 || md.n_tri_index < 0) return "negative count";
-  if (nt > 0x3fffffffLL || md.n_nodes > 0x3fffffffLL || md.n_tri_index > 0x3fffffffLL)
-    return "mesh too large";
+  if (nt > RTB_MAX_PRIMS) return "mesh too large: more than 2^29 triangles";
+  if (md.n_nodes > 0x3fffffffLL || md.n_tri_index > 0x3fffffffLL) return "mesh too large";
   if ((nt > 0 && !md.vertices) || (md.n_nodes > 0 && !md.nodes) || (md.n_tri_index > 0 && !md.tri_index))
     return "null mesh array";
   std::vector<double2> nodes((size_t)md.n_nodes * 4);
@@ -1241,7 +1241,7 @@ rt_status do_upload(rt_ctx* ctx, const rt_scene_desc* d, rt_scene** out,
       std::vector<int32_t> order;
       // leaves of 4 spheres: 47.6 ms for the 1,000-sphere ring frame (1080p,
       // 4 spp) against 49.4 ms with 8 or 12
-      build_bvh(bmin, bmax, 4, 1e-6 * (1.0 + scale), &bn, &order);
+      build_bvh(bmin, bmax, RTB_LEAF, 1e-6 * (1.0 + scale), &bn, &order);
       std::vector<float4> fbvh;
       put_fbvh(bn, &fbvh);  // the walks test single-precision boxes only
       DSphGroup G{};
