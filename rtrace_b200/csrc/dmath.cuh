@@ -271,7 +271,7 @@ struct StdRng {
 #define RTB_LEAF 4
 #define RTB_MAX_PRIMS (1 << 29)
 #define RTB_WALK_DONE 0x7fffffff
-RTB_HD int walk_ref(int idx, int cnt) { return cnt ? ~(idx << 2 | (cnt - 1)) : idx; }
+RTB_HD int walk_ref(int idx, int cnt) { return cnt ? (int)(0u - (4u * (unsigned)idx + (unsigned)cnt)) : idx; }
 RTB_HD int leaf_first(int ref) { return ~ref >> 2; }
 RTB_HD int leaf_count(int ref) { return (~ref & 3) + 1; }
 
