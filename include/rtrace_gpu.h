@@ -630,6 +630,10 @@ rt_status rt_debug_mesh_hit(rt_ctx* ctx, const rt_scene* scene, int32_t object_i
  * device's conversion against the host's, which host-prepared uploads
  * copy) differs.  More than 4 triangles (the BVH leaf size). */
 rt_status rt_debug_mesh_prep(rt_ctx* ctx, const rt_mesh_desc* mesh, uint32_t* mismatch);
+/* Nanoseconds without any progress after which the context's frames give up
+ * a wait between the stages of the queue levels that share a launch
+ * (RT_ERR_DEVICE_WATCHDOG); 0: the default, 20 seconds. */
+rt_status rt_debug_set_barrier_limit(rt_ctx* ctx, int64_t ns);
 
 #ifdef __cplusplus
 }

@@ -303,6 +303,13 @@ __device__ __forceinline__ int walk_lanes(const DScene& S, long long n, int nblk
   return lanes;
 }
 
+// A step of a stage is done: a warp's rays are traced, a light's cones walked
+// or a round of its samples taken.  Counted for the waits of k_levels' grid
+// barrier; the stages' own launches pass no counter.
+__device__ __forceinline__ void step_done(unsigned* steps) {
+  if (steps && (threadIdx.x & 31) == 0) atomicAdd(steps, 1u);
+}
+
 // Level 0 walks its rays in tiles of pixels (tile_place) from this many up:
 // a warp's walks then share more of their nodes.  4K terrain 11.98 -> 11.18
 // ms (trace 3.48 -> 3.05, cones 3.39 -> 3.08; with tiles 16 x 2 11.52), 2560x1440
@@ -325,7 +332,7 @@ __device__ __forceinline__ int primary_place(const DFrame& F, int i) {
 // 3.05 in tiles, TILED_RAYS).
 // --------------------------------------------------------------------------
 template <bool COUNT>
-__device__ __forceinline__ void trace_body(const DFrame& F, int level, int bid, int nblk) {
+__device__ __forceinline__ void trace_body(const DFrame& F, int level, int bid, int nblk, unsigned* steps = nullptr) {
   int n = F.counts[level];
   RayBuf q = F.q[level & 1];
   LevelBuf L = F.levels[level];
@@ -369,6 +376,7 @@ __device__ __forceinline__ void trace_body(const DFrame& F, int level, int bid, 
       F.ht[slot] = h.t;
       F.hit_ray[slot] = i;
     }
+    step_done(steps);
   }
   if (COUNT) flush_work(F, w, 0);
 }
@@ -533,7 +541,8 @@ __device__ __forceinline__ bool next_offset(StdRng& rng, double radius, double* 
 // 1,000-sphere frame 0.3 ms.
 #define SPLIT_PAIRS (1 << 17)
 template <bool COUNT, bool SPLIT>
-__device__ __forceinline__ void shaft_body(const DFrame& F, int level, long long c0, int bid, int nblk) {
+__device__ __forceinline__ void shaft_body(const DFrame& F, int level, long long c0, int bid, int nblk,
+                                           unsigned* steps = nullptr) {
   __shared__ int2 s_cand[RTB_CAND][128];
   const DScene& S = F.S;
   const long long nh = F.nhits[level];
@@ -632,6 +641,7 @@ __device__ __forceinline__ void shaft_body(const DFrame& F, int level, long long
         for (int j = 0; j < nc; j++) F.pair.cand[(size_t)st * RTB_CAND + j] = s_cand[j][threadIdx.x];
       }
       if (active) F.pair.st[li * F.chunk_hits + hl] = st;
+      step_done(steps);
     }
     unsigned lit = 0;
     if (shaded && pairing && active)
@@ -713,7 +723,7 @@ __device__ __forceinline__ int part_tasks(const DFrame& F) {
 // Warp w of nw takes the class's tasks w, w + nw, ...
 template <int KIND, bool COUNT>
 __device__ __forceinline__ void part_body(const DFrame& F, int level, long long c0, PartShared& sm, long long w0,
-                                          long long nw) {
+                                          long long nw, unsigned* steps) {
   constexpr int NL = KIND == PART_LIT2 ? 2 : 1;  // lights of an entry
   constexpr bool LIT = KIND == PART_LIT || KIND == PART_LIT2;
   const unsigned FULL = 0xffffffffu;
@@ -770,6 +780,7 @@ __device__ __forceinline__ void part_body(const DFrame& F, int level, long long 
     for (int u = 0; u < NL; u++) tot[u] = mk(0.0, 0.0, 0.0);
     int got = 0, visible = 0, rounds = 0;  // offsets drawn, unblocked samples, ChaCha rounds
     for (int s0 = 0; s0 < dsamp; s0 += g) {
+      step_done(steps);
       const int need = min(dsamp, s0 + g);
       // Draw until every group holds its next samples.  A lane that draws
       // while others wait costs nothing, so groups draw ahead whenever the
@@ -903,7 +914,8 @@ __device__ __forceinline__ void part_body(const DFrame& F, int level, long long 
 // beside them.  A grid whose blocks are all resident (k_levels) goes through
 // the queues' tasks as one sequence.
 template <bool COUNT>
-__device__ __forceinline__ void part_all(const DFrame& F, int level, long long c0, int bid, int nblk, bool resident) {
+__device__ __forceinline__ void part_all(const DFrame& F, int level, long long c0, int bid, int nblk, bool resident,
+                                         unsigned* steps = nullptr) {
   __shared__ PartShared sm;
   const int wid = threadIdx.x >> 5;
   // a learned level 0 takes the lit pairs' shading from the network
@@ -918,13 +930,13 @@ __device__ __forceinline__ void part_all(const DFrame& F, int level, long long c
   // the warp's first task of a class that follows `tasks` others
   auto next = [&](int tasks) { w0 = (w0 + nw - tasks % nw) % nw; };
   auto mine = [&](int k) { return part < 0 || part == k ? w0 : none; };
-  part_body<PART_WALK, COUNT>(F, level, c0, sm, mine(0), nw);
+  part_body<PART_WALK, COUNT>(F, level, c0, sm, mine(0), nw, steps);
   if (part < 0) next(part_tasks<PART_WALK>(F));
-  part_body<PART_LIST, COUNT>(F, level, c0, sm, mine(1), nw);
+  part_body<PART_LIST, COUNT>(F, level, c0, sm, mine(1), nw, steps);
   if (part < 0) next(part_tasks<PART_LIST>(F));
-  part_body<PART_LIT2, COUNT>(F, level, c0, sm, lit ? mine(2) : none, nw);
+  part_body<PART_LIT2, COUNT>(F, level, c0, sm, lit ? mine(2) : none, nw, steps);
   if (part < 0) next(part_tasks<PART_LIT2>(F));
-  part_body<PART_LIT, COUNT>(F, level, c0, sm, lit ? mine(3) : none, nw);
+  part_body<PART_LIT, COUNT>(F, level, c0, sm, lit ? mine(3) : none, nw, steps);
 }
 template <bool COUNT>
 __global__ void __launch_bounds__(128, 4) k_part(const __grid_constant__ DFrame F, int level, long long c0) {
@@ -1316,24 +1328,34 @@ __global__ void k_pixels_multi(const DFrame* __restrict__ T, const int* __restri
 //
 // The barrier: the blocks are co-resident (cooperative launch), bar[0]
 // counts their arrivals and each stage waits for the next multiple of the
-// grid.  A block that waited 20 seconds sets the watchdog's error and leaves,
-// and so, at their next barrier, do the others.
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned* target, int* err) {
+// grid.  A stage may last as long as its work takes: a block waits on while
+// others arrive or do steps (bar[2], step_done).  One that sees neither for
+// `limit` nanoseconds sets the watchdog's error and leaves, and so, at their
+// next barrier, do the others.  A step is one walk of the scene at most, and
+// the host admits scenes only where that is far shorter (kCoopWalk).
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned* target, unsigned long long limit, int* err) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
+    volatile unsigned* vb = bar;
     *target += gridDim.x;
     __threadfence();
     atomicAdd(bar, 1u);
     unsigned long long t0, t;
+    unsigned seen = vb[0] + vb[2];
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
     bool ok = true;
-    while ((int)(*(volatile unsigned*)bar - *target) < 0) {
+    while ((int)(vb[0] - *target) < 0) {
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-      if (t - t0 > 20000000000ull) {
-        atomicOr(err, ERR_BARRIER);
-        ok = false;
-        break;
+      if (t - t0 > limit) {
+        const unsigned now = vb[0] + vb[2];
+        if (now == seen) {
+          atomicOr(err, ERR_BARRIER);
+          ok = false;
+          break;
+        }
+        seen = now;
+        t0 = t;
       }
     }
     __threadfence();
@@ -1342,23 +1364,25 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned* target, in
   __syncthreads();
   return s_ok != 0;
 }
-__global__ void __launch_bounds__(128, 4) k_levels(const __grid_constant__ DFrame F, int first, int levels, unsigned* bar) {
+__global__ void __launch_bounds__(128, 4) k_levels(const __grid_constant__ DFrame F, int first, int levels, unsigned* bar,
+                                                     unsigned long long limit) {
   const int bid = blockIdx.x, nblk = gridDim.x;
   unsigned target = 0;
+  unsigned* steps = bar + 2;
   bool ok = true;
   for (int l = first; ok && l < levels; l++) {
     if (*(volatile int*)&F.counts[l] == 0) break;
-    trace_body<false>(F, l, bid, nblk);
-    if (!(ok = grid_barrier(bar, &target, F.err))) break;
+    trace_body<false>(F, l, bid, nblk, steps);
+    if (!(ok = grid_barrier(bar, &target, limit, F.err))) break;
     if (*(volatile int*)&F.nhits[l] == 0) break;
-    shaft_body<false, true>(F, l, 0, bid, nblk);
-    if (!(ok = grid_barrier(bar, &target, F.err))) break;
+    shaft_body<false, true>(F, l, 0, bid, nblk, steps);
+    if (!(ok = grid_barrier(bar, &target, limit, F.err))) break;
     if (*(volatile int*)&F.pair.n[0] + *(volatile int*)&F.pair.n[1] + *(volatile int*)&F.pair.n[2] + *(volatile int*)&F.pair.n[3] > 0) {
-      part_all<false>(F, l, 0, bid, nblk, true);
-      if (!(ok = grid_barrier(bar, &target, F.err))) break;
+      part_all<false>(F, l, 0, bid, nblk, true, steps);
+      if (!(ok = grid_barrier(bar, &target, limit, F.err))) break;
     }
     light_body(F, l, 0, bid, nblk);
-    if (!(ok = grid_barrier(bar, &target, F.err))) break;
+    if (!(ok = grid_barrier(bar, &target, limit, F.err))) break;
   }
   if (ok) fold_body(F, bid, nblk);
   // the last block to leave clears the barrier for the next launch

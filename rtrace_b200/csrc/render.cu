@@ -76,6 +76,7 @@ struct rt_scene {
   std::vector<int> obj_kind, obj_mesh;  // per World object
   int n_point_lights = 0, n_disk_lights = 0;
   int n_reflecting = 0;  // objects of a reflecting material
+  long long walk_tests = 0;  // objects, triangles and k-d leaf entries of all World objects
   // upload arena: one device block; small arrays are staged in the
   // context's pinned buffer, mesh arrays copied from their own host memory
   char* blk = nullptr;
@@ -112,6 +113,8 @@ struct FrameResult {
 // with the counts, hits, counters and error word copied one by one too).
 // Larger images gain nothing: the driver's own staging is as fast.
 constexpr size_t kPinImage = 1 << 20;
+// A wait of k_levels' grid barrier gives up when nothing moved for this long.
+const long long kBarrierNs = 20000000000LL;
 
 struct rt_ctx {
   int device = 0;
@@ -137,6 +140,7 @@ struct rt_ctx {
   unsigned long long* d_stats = nullptr;
   int* d_err = nullptr;
   unsigned* d_bar = nullptr;  // k_levels' grid barrier
+  long long barrier_ns = kBarrierNs;
   int level_blocks = 0;       // blocks of k_levels that are resident together
   // learned soft shadows: network and its buffers (grown on demand)
   DenoiseNet net;
@@ -235,6 +239,11 @@ const long long kPairCap = 1LL << 26;
 constexpr int kCoopLevel = 2;
 const long long kSmallFrame = 1LL << 22;
 constexpr int kFewReflecting = 4;
+// And the most that one walk may test: objects, triangles and k-d leaf
+// entries.  A ray that opens every box of a mesh takes 0.6 us per triangle
+// (1.15 s on two million), so that one step of a stage ends in seconds,
+// whatever the rays, where a barrier waits kBarrierNs for it.
+const long long kCoopWalk = 1LL << 23;
 
 rt_status ensure_scratch(rt_ctx* ctx, long long n_rays, int levels, long long n_pix, long long n_hits,
                          long long n_pairs, long long n_disk) {
@@ -299,7 +308,7 @@ rt_status ensure_scratch(rt_ctx* ctx, long long n_rays, int levels, long long n_
     take(&F.mask, P);
     take(&F.rgb, 3 * P);
     take(&ctx->d_res, 1);
-    take(&ctx->d_bar, 2);
+    take(&ctx->d_bar, 4);
     if (pass == 0) CK(dalloc(ctx->scratch, &block, used));
   }
   // on the stream of the kernels that read them: it does not wait for the
@@ -307,7 +316,7 @@ rt_status ensure_scratch(rt_ctx* ctx, long long n_rays, int levels, long long n_
   // could land in a running k_levels' arrival count
   CK(cudaMemcpyAsync(ctx->d_levels, ctx->h_levels.data(), (Lv + 1) * sizeof(LevelBuf), cudaMemcpyHostToDevice,
                      ctx->stream));
-  CK(cudaMemsetAsync(ctx->d_bar, 0, 2 * sizeof(unsigned), ctx->stream));
+  CK(cudaMemsetAsync(ctx->d_bar, 0, 4 * sizeof(unsigned), ctx->stream));
   ctx->d_counts = ctx->d_res->counts;
   ctx->d_nhits = ctx->d_res->nhits;
   ctx->d_stats = ctx->d_res->stats;
@@ -1293,8 +1302,10 @@ rt_status do_upload(rt_ctx* ctx, const rt_scene_desc* d, rt_scene** out,
     M.cb_shininess = m.checker_shininess;
   }
   for (int i = 0; i < d->n_objects; i++) {
-    const int m = d->objects[i].material;
+    const rt_object_desc& o = d->objects[i];
+    const int m = o.material;
     if (m >= 0 && m < d->n_materials && mats[m].has_refl && mats[m].refl > 0.0) sc->n_reflecting++;
+    sc->walk_tests += o.kind == RT_OBJ_MESH ? d->meshes[o.mesh].n_triangles + d->meshes[o.mesh].n_tri_index : 1;
   }
   std::vector<DLight> lights(d->n_lights);
   int K = 0;
@@ -1644,12 +1655,13 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
   // 1080p x 4: 18.4 ms; 19.3 with k_levels) the stages' own grids and
   // register budgets do the deep levels' work faster.  Not beside other
   // streams of the same call (batch lanes): a cooperative grid waits until
-  // all its blocks find room.  Nor where a stage could outlast the barrier's
-  // limit: `tests` bounds its object tests.
+  // all its blocks find room.  Nor in scenes where one walk alone could
+  // outlast the barrier's limit (kCoopWalk), nor for frames of so many rays
+  // that the launches are nothing beside their work.
   const double rays0 = (double)nprim * (1.0 + K_full);
   int first_coop = levels;
   if (!ctx->borrowed_net && !count && !Lc.timed && levels > kCoopLevel && chunk >= nprim &&
-      rays0 * std::max(1, sc->S.n_obj) < (double)(1LL << 35) &&
+      sc->walk_tests <= kCoopWalk && rays0 * std::max(1, sc->S.n_obj) < (double)(1LL << 35) &&
       (rays0 <= (double)kSmallFrame || sc->n_reflecting <= kFewReflecting))
     first_coop = kCoopLevel;
   if (first_coop < levels && !ctx->level_blocks) {
@@ -1737,7 +1749,8 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
         F.lanes_log2 = pair_lanes_log2(dsamp);
         int first = first_coop, nl = levels;
         unsigned* bar = ctx->d_bar;
-        void* args[] = {&F, &first, &nl, &bar};
+        unsigned long long limit = (unsigned long long)ctx->barrier_ns;
+        void* args[] = {&F, &first, &nl, &bar, &limit};
         const int grid = (int)std::min<long long>(
             ctx->level_blocks, std::max((nprim + 15) / 16, ((nprim * std::max(1, sc->n_disk_lights) << F.lanes_log2) + 127) / 128));
         CK(cudaLaunchCooperativeKernel((const void*)k_levels, dim3(grid), dim3(128), args, 0, s));
@@ -1770,7 +1783,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
     };
     put(&F, sizeof F);
     const long long kl[] = {nprim, npix, chunk, levels, max_depth, sc->n_disk_lights, lrays, dsamp, learned, count,
-                            nsm, spp, H, W, (long long)o_shm, fallback, fb_dsamp, first_coop};
+                            nsm, spp, H, W, (long long)o_shm, fallback, fb_dsamp, first_coop, ctx->barrier_ns};
     put(kl, sizeof kl);
     if (learned) {
       const void* ap[] = {ctx->d_dn_arena};
@@ -1842,7 +1855,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
   if (herr & ERR_RANGE_OVERFLOW) return fail(ctx, RT_ERR_RENDER, "UniformSampler::sample_single: range overflow");
   if (herr & DN_ERR_WAIT) return fail(ctx, RT_ERR_DEVICE_WATCHDOG, "denoiser: a tensor-core wait timed out");
   if (herr & ERR_BARRIER) {
-    cudaMemsetAsync(ctx->d_bar, 0, 2 * sizeof(unsigned), s);
+    cudaMemsetAsync(ctx->d_bar, 0, 4 * sizeof(unsigned), s);
     return fail(ctx, RT_ERR_DEVICE_WATCHDOG, "a grid barrier timed out");
   }
   if (herr & (ERR_WATCHDOG | ERR_STACK))
@@ -2997,6 +3010,12 @@ rt_status rt_debug_mesh_prep(rt_ctx* ctx, const rt_mesh_desc* md, uint32_t* mism
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "mesh preparation check");
   *mismatch = m;
   ctx->err.clear();
+  return RT_OK;
+}
+
+rt_status rt_debug_set_barrier_limit(rt_ctx* ctx, int64_t ns) {
+  if (!ctx || ns < 0) return fail(ctx, RT_ERR_INVALID_ARGUMENT, "bad argument");
+  ctx->barrier_ns = ns ? ns : kBarrierNs;
   return RT_OK;
 }
 
