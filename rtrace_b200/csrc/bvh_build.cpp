@@ -135,12 +135,20 @@ struct Builder {
 // Binned SAH build: 16 centroid bins per axis; a node splits at the bin
 // boundary with the smallest (left area x count + right area x count), the
 // first such on axis x, y, z in that order; a node whose centroids cannot
-// be binned apart splits at its median primitive id.  Leaves hold at most
+// be binned apart splits at its median primitive id, and so does what is
+// left where the tree would exceed kBvhLevels (primitives that shrink
+// towards a point are peeled off a few per level).  Leaves hold at most
 // `leaf` primitives.  The split sets depend only on the primitives, never
 // on their order, so the tree is deterministic.
 struct SahBuilder {
   int leaf;
   double pad;
+  // Levels of nodes that median splits make of n primitives.
+  int median_levels(int n) const {
+    int levels = 0;
+    for (; n > leaf; n -= n / 2) levels++;
+    return levels;
+  }
   static double area(const double mn[3], const double mx[3]) {
     const double dx = mx[0] - mn[0], dy = mx[1] - mn[1], dz = mx[2] - mn[2];
     return dx * dy + dy * dz + dz * dx;
@@ -169,9 +177,12 @@ struct SahBuilder {
     constexpr int B = 16;
     double best = inf;
     int best_axis = -1, best_b = -1;
+    // a median split leaves its subtree one level less, so no level follows
+    // the last one
+    const bool deep = depth + median_levels(n) >= kBvhLevels;
     for (int a = 0; a < 3; a++) {
       const double ext = cmax[a] - cmin[a];
-      if (!(ext > 0)) continue;
+      if (deep || !(ext > 0)) continue;
       int cnt[B] = {};
       double bmn[B][3], bmx[B][3];
       for (int b = 0; b < B; b++)

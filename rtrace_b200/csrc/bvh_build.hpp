@@ -34,6 +34,10 @@ struct BvhNode {
 void build_bvh(const std::vector<double>& bmin, const std::vector<double>& bmax, int leaf_size, double pad,
                std::vector<BvhNode>* nodes, std::vector<int32_t>* order);
 
+// Levels of nodes that either build makes at most (median splits reach 27 on
+// the largest accepted mesh): a walk's stack holds one entry per level.
+constexpr int kBvhLevels = 60;
+
 // The same interface, layout and leaf order, with each node split at the
 // boundary of 16 centroid bins (per axis) that minimises the children's
 // surface area times primitive count: fewer node visits per ray than the

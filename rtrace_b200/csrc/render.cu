@@ -799,6 +799,7 @@ void parallel_ranges(long long n, F f) {
 // fastest on the 82k-triangle mesh frame (7.21 ms; 2: 7.31, 3: 7.26,
 // 5: 7.28, 6: 7.30, 8: 7.39, 12: 7.68); with double boxes it was 8.
 const int kMeshLeaf = RTB_LEAF;
+static_assert(kBvhLevels <= RTB_STACK, "a walk pushes a child per level");
 // Meshes from this many triangles up are prepared on the device (median
 // split BVH, tens of ms for millions of triangles); smaller ones on the
 // host with a binned SAH BVH (about 7% fewer node visits per ray, 4% on the
