@@ -116,6 +116,12 @@ constexpr size_t kPinImage = 1 << 20;
 // A wait of k_levels' grid barrier gives up when nothing moved for this long.
 const long long kBarrierNs = 20000000000LL;
 
+// What sizes a frame's scratch: primary rays, queue levels, pixels, and the
+// hits, (hit, light) pairs and (hit, disk light) pairs held at once.
+struct ScratchDims {
+  long long rays, levels, pixels, hits, pairs, disk;
+};
+
 struct rt_ctx {
   int device = 0;
   int num_sms = 148;
@@ -123,12 +129,7 @@ struct rt_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<cudaEvent_t> stage_ev;
   std::string err;
-  long long cap_rays = 0;
-  int cap_levels = 0;
-  long long cap_pixels = 0;
-  long long cap_pairs = 0;  // (hit, light) pairs
-  long long cap_disk = 0;   // (hit, disk light) pairs
-  long long cap_hits = 0;   // hit records
+  ScratchDims cap{};
   std::vector<void*> scratch;
   DFrame F{};
   std::vector<LevelBuf> h_levels;
@@ -229,10 +230,11 @@ const size_t kMaxGraphs = 256;
 // Shadow rays of one frame of a batch's fused group at most, and of the
 // learned pass (which holds a whole frame's hits).
 const long long kShadowCap = 1LL << 28;
-// (hit, light) pairs kept on the device at once: 32 bytes each, 97 more for
-// a disk light's (mostly its candidates), 8.7 GB at most.  A 4K frame with 4 samples
-// and two lights fits in one chunk per level: chunks beyond a level's hits
-// still cost their launches.
+// (hit, light) pairs kept on the device at once: 32 bytes each, 57 more for
+// a disk light's (queue entries and three candidates), 6 GB at most; a
+// learned frame holds all of its hits' pairs, whose rays kShadowCap limits.
+// A 4K frame with 4 samples and two lights fits in one chunk per level:
+// chunks beyond a level's hits still cost their launches.
 const long long kPairCap = 1LL << 26;
 // The first queue level of k_levels, and the frames it serves: at most this
 // many camera and shadow rays at the primary level, or objects that reflect.
@@ -245,26 +247,15 @@ constexpr int kFewReflecting = 4;
 // whatever the rays, where a barrier waits kBarrierNs for it.
 const long long kCoopWalk = 1LL << 23;
 
-rt_status ensure_scratch(rt_ctx* ctx, long long n_rays, int levels, long long n_pix, long long n_hits,
-                         long long n_pairs, long long n_disk) {
-  if (n_rays <= ctx->cap_rays && levels <= ctx->cap_levels && n_pix <= ctx->cap_pixels && n_hits <= ctx->cap_hits &&
-      n_pairs <= ctx->cap_pairs && n_disk <= ctx->cap_disk)
-    return RT_OK;
-  CK(cudaStreamSynchronize(ctx->stream));
-  long long R = std::max(n_rays, ctx->cap_rays);
-  int Lv = std::max(levels, ctx->cap_levels);
-  long long P = std::max(n_pix, ctx->cap_pixels);
-  const long long HS = std::max(n_hits, ctx->cap_hits), PS = std::max(n_pairs, ctx->cap_pairs);
-  const long long DS = std::max(n_disk, ctx->cap_disk);
-  drop_graphs(ctx);
-  free_all(ctx->scratch);
-  ctx->cap_rays = ctx->cap_levels = 0;
-  ctx->cap_pixels = ctx->cap_hits = ctx->cap_pairs = ctx->cap_disk = 0;
-  DFrame& F = ctx->F;
-  // One block for all of them, laid out by two passes of the same code: a
-  // cudaMalloc (and, when the scratch grows, a cudaFree) apiece cost a first
-  // render of a batch's lanes seconds, as they queue on one device.
-  char* block = nullptr;
+struct ScratchHead {
+  LevelBuf* levels;
+  FrameResult* res;
+  unsigned* bar;
+};
+// Lays the scratch out in one block and returns its bytes; block null: the
+// bytes only.  (A cudaMalloc and, when the scratch grows, a cudaFree per array
+// cost a first render of a batch's lanes seconds, as they queue on one device.)
+size_t lay_scratch(char* block, const ScratchDims& d, DFrame& F, std::vector<LevelBuf>& levels, ScratchHead& head) {
   size_t used = 0;
   auto take = [&](auto** ptr, long long count) {
     typedef std::remove_reference_t<decltype(**ptr)> T;
@@ -272,50 +263,68 @@ rt_status ensure_scratch(rt_ctx* ctx, long long n_rays, int levels, long long n_
     *ptr = block ? reinterpret_cast<T*>(block + used) : nullptr;
     used += std::max(1LL, count) * sizeof(T);
   };
-  for (int pass = 0; pass < 2; pass++) {
-    used = 0;
-    for (int k = 0; k < 2; k++) {
-      take(&F.q[k].ox, R); take(&F.q[k].oy, R); take(&F.q[k].oz, R);
-      take(&F.q[k].dx, R); take(&F.q[k].dy, R); take(&F.q[k].dz, R);
-      take(&F.q[k].seed, R);
-    }
-    take(&F.hobj, R); take(&F.haux, R); take(&F.hent, R); take(&F.ht, R);
-    take(&F.hit_ray, R);
-    ctx->h_levels.assign(Lv + 1, LevelBuf{});
-    for (int l = 0; l < Lv; l++) {
-      LevelBuf& L = ctx->h_levels[l];
-      take(&L.r, R); take(&L.g, R); take(&L.b, R);
-      take(&L.refl, R); take(&L.child, R);
-    }
-    take(&ctx->d_levels, Lv + 1);
-    HitBuf& B = F.hr;
-    take(&B.px, HS); take(&B.py, HS); take(&B.pz, HS);
-    take(&B.nx, HS); take(&B.ny, HS); take(&B.nz, HS);
-    take(&B.u, HS); take(&B.v, HS); take(&B.mat, HS);
-    PairBuf& Q = F.pair;
-    take(&Q.st, PS); take(&Q.vis, PS);
-    for (int k = 0; k < 3; k++) take(&Q.sum[k], PS);
-    for (int k = 0; k < 4; k++) take(&Q.queue[k], DS);
-    take(&Q.cand, DS * RTB_CAND); take(&Q.ncand, DS);
-    take(&Q.n, 8);
-    take(&F.pdepth, R); take(&F.pnx, R); take(&F.pny, R); take(&F.pnz, R);
-    take(&F.phit, R);
-    take(&F.pobj, R);
-    take(&F.cr, P); take(&F.cg, P); take(&F.cb, P);
-    take(&F.dep, P); take(&F.nx, P); take(&F.ny, P); take(&F.nz, P);
-    take(&F.valid, P);
-    take(&F.oid, P);
-    take(&F.mask, P);
-    take(&F.rgb, 3 * P);
-    take(&ctx->d_res, 1);
-    take(&ctx->d_bar, 4);
-    if (pass == 0) CK(dalloc(ctx->scratch, &block, used));
+  const long long R = d.rays, P = d.pixels;
+  for (int k = 0; k < 2; k++) {
+    take(&F.q[k].ox, R); take(&F.q[k].oy, R); take(&F.q[k].oz, R);
+    take(&F.q[k].dx, R); take(&F.q[k].dy, R); take(&F.q[k].dz, R);
+    take(&F.q[k].seed, R);
   }
+  take(&F.hobj, R); take(&F.haux, R); take(&F.hent, R); take(&F.ht, R);
+  take(&F.hit_ray, R);
+  levels.assign(d.levels + 1, LevelBuf{});
+  for (long long l = 0; l < d.levels; l++) {
+    LevelBuf& L = levels[l];
+    take(&L.r, R); take(&L.g, R); take(&L.b, R);
+    take(&L.refl, R); take(&L.child, R);
+  }
+  take(&head.levels, d.levels + 1);
+  HitBuf& B = F.hr;
+  take(&B.px, d.hits); take(&B.py, d.hits); take(&B.pz, d.hits);
+  take(&B.nx, d.hits); take(&B.ny, d.hits); take(&B.nz, d.hits);
+  take(&B.u, d.hits); take(&B.v, d.hits); take(&B.mat, d.hits);
+  PairBuf& Q = F.pair;
+  take(&Q.st, d.pairs); take(&Q.vis, d.pairs);
+  for (int k = 0; k < 3; k++) take(&Q.sum[k], d.pairs);
+  for (int k = 0; k < 4; k++) take(&Q.queue[k], d.disk);
+  take(&Q.cand, d.disk * RTB_CAND); take(&Q.ncand, d.disk);
+  take(&Q.n, 8);
+  take(&F.pdepth, R); take(&F.pnx, R); take(&F.pny, R); take(&F.pnz, R);
+  take(&F.phit, R);
+  take(&F.pobj, R);
+  take(&F.cr, P); take(&F.cg, P); take(&F.cb, P);
+  take(&F.dep, P); take(&F.nx, P); take(&F.ny, P); take(&F.nz, P);
+  take(&F.valid, P);
+  take(&F.oid, P);
+  take(&F.mask, P);
+  take(&F.rgb, 3 * P);
+  take(&head.res, 1);
+  take(&head.bar, 4);
+  return used;
+}
+
+rt_status ensure_scratch(rt_ctx* ctx, const ScratchDims& n) {
+  if (n.rays <= ctx->cap.rays && n.levels <= ctx->cap.levels && n.pixels <= ctx->cap.pixels && n.hits <= ctx->cap.hits &&
+      n.pairs <= ctx->cap.pairs && n.disk <= ctx->cap.disk)
+    return RT_OK;
+  CK(cudaStreamSynchronize(ctx->stream));
+  const ScratchDims& c = ctx->cap;
+  const ScratchDims d{std::max(n.rays, c.rays), std::max(n.levels, c.levels), std::max(n.pixels, c.pixels),
+                      std::max(n.hits, c.hits), std::max(n.pairs, c.pairs), std::max(n.disk, c.disk)};
+  drop_graphs(ctx);
+  free_all(ctx->scratch);
+  ctx->cap = ScratchDims{};
+  ScratchHead head;
+  char* block = nullptr;
+  CK(dalloc(ctx->scratch, &block, lay_scratch(nullptr, d, ctx->F, ctx->h_levels, head)));
+  lay_scratch(block, d, ctx->F, ctx->h_levels, head);
+  ctx->d_levels = head.levels;
+  ctx->d_res = head.res;
+  ctx->d_bar = head.bar;
   // on the stream of the kernels that read them: it does not wait for the
   // legacy stream, and a clear queued there behind another thread's work
   // could land in a running k_levels' arrival count
-  CK(cudaMemcpyAsync(ctx->d_levels, ctx->h_levels.data(), (Lv + 1) * sizeof(LevelBuf), cudaMemcpyHostToDevice,
-                     ctx->stream));
+  CK(cudaMemcpyAsync(ctx->d_levels, ctx->h_levels.data(), ctx->h_levels.size() * sizeof(LevelBuf),
+                     cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(ctx->d_bar, 0, 4 * sizeof(unsigned), ctx->stream));
   ctx->d_counts = ctx->d_res->counts;
   ctx->d_nhits = ctx->d_res->nhits;
@@ -323,12 +332,7 @@ rt_status ensure_scratch(rt_ctx* ctx, long long n_rays, int levels, long long n_
   ctx->d_err = &ctx->d_res->err;
   ctx->d_fbn = ctx->d_res->fbn;
   if (!ctx->pin_res) CK(cudaMallocHost((void**)&ctx->pin_res, sizeof(FrameResult) + kPinImage));
-  ctx->cap_rays = R;
-  ctx->cap_levels = Lv;
-  ctx->cap_pixels = P;
-  ctx->cap_hits = HS;
-  ctx->cap_pairs = PS;
-  ctx->cap_disk = DS;
+  ctx->cap = d;
   return RT_OK;
 }
 
@@ -1530,7 +1534,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
   if (learned && std::max(1LL, kShadowCap / K_0) < nprim)
     return fail(ctx, RT_ERR_INVALID_ARGUMENT, "too many primary samples for learned shadows in one pass");
   const long long chunk = learned || !n_lights ? nprim : std::max(1LL, std::min(nprim, kPairCap / n_lights));
-  rt_status st = ensure_scratch(ctx, nprim, levels, npix, chunk, chunk * n_lights, chunk * sc->n_disk_lights);
+  rt_status st = ensure_scratch(ctx, {nprim, levels, npix, chunk, chunk * n_lights, chunk * sc->n_disk_lights});
   if (st != RT_OK) return st;
   if (learned || want_aov) {
     st = ensure_dn_scratch(ctx, nprim);
@@ -2589,7 +2593,7 @@ rt_status rt_render_batch(rt_ctx* ctx, rt_job* jobs, uint32_t n, uint32_t lanes,
   std::vector<double> cost(n, 0.0);
   std::vector<uint32_t> fused;
   std::vector<char> in_group(n, 0);
-  std::vector<double> scratch(n, 0.0);  // estimated scratch bytes of a fused frame
+  std::vector<double> scratch(n, 0.0);  // scratch bytes of a fused frame
   for (uint32_t i = 0; i < n; i++) {
     const rt_render_params& P = jobs[i].params;
     const rt_scene* sc = jobs[i].scene;
@@ -2608,17 +2612,17 @@ rt_status rt_render_batch(rt_ctx* ctx, rt_job* jobs, uint32_t n, uint32_t lanes,
         !P.learned_shadows && !outline && P.max_depth > 0 && P.max_depth <= RTB_MAX_LEVELS && P.samples > 0 &&
         !(P.flags & (RT_FLAG_STAGE_TIMES | RT_FLAG_COUNT_WORK)) && nprim * std::max(K, 1.0) <= (double)kShadowCap &&
         nprim * nl <= (double)kPairCap) {
-      // a fused frame keeps all its scratch at once: per primary ray the
-      // queues, hit records, per-level colours and outline data, the shading
-      // record (68 bytes) and pairs (32 bytes per light, 97 per disk light),
-      // and about 80 bytes per pixel
-      const double levels = std::max(1, std::min(P.max_depth, RTB_MAX_LEVELS));
-      scratch[i] = nprim * (173.0 + 36.0 * levels + 68.0 + 32.0 * nl + 97.0 * sc->n_disk_lights) +
-                   (double)P.width * P.height * 80.0;
+      // a fused frame keeps all its scratch at once, every hit's pairs with it
+      const long long n = (long long)nprim, nd = sc->n_disk_lights;
+      DFrame F;
+      std::vector<LevelBuf> lv;
+      ScratchHead head;
+      scratch[i] = (double)lay_scratch(nullptr, {n, P.max_depth, (long long)P.width * P.height, n, n * (long long)nl, n * nd},
+                                       F, lv, head);
       fused.push_back(i);
     }
   }
-  // the smallest frames first, while the estimated scratch fits the budget
+  // the smallest frames first, while their scratch fits the budget
   std::stable_sort(fused.begin(), fused.end(), [&](uint32_t a, uint32_t b) { return scratch[a] < scratch[b]; });
   {
     double used = 0.0;
@@ -2840,7 +2844,7 @@ rt_status rt_denoiser_run(rt_ctx* ctx, const uint16_t* features, uint32_t planes
   if (st != RT_OK) return st;
   // the scratch error word is shared with renders on this context
   if (!ctx->d_err) {
-    st = ensure_scratch(ctx, 1, 1, 1, 1, 1, 1);
+    st = ensure_scratch(ctx, {1, 1, 1, 1, 1, 1});
     if (st != RT_OK) return st;
   }
   CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));

@@ -1,5 +1,5 @@
 """A context's scratch memory: set up in the order of the stream whose kernels
-use it."""
+use it, and counted for a batch's group as it is allocated."""
 import os
 import re
 
@@ -46,3 +46,33 @@ def test_first_frames_beside_a_busy_legacy_stream(gpu_ctx, tmp_path):
             assert np.array_equal(rt.Renderer(w, h).render(scene), want[w])
         scene.close()
     torch.cuda.synchronize()
+
+
+# a budget for four frames of a group holds four: per primary ray and level 36
+# bytes, 241 more (queues, hits, records, outline), 32 per light and 57 per
+# disk light; per pixel 80
+@pytest.mark.gpu
+@pytest.mark.parametrize("disk,point", [(0, 1), (2, 0), (3, 1)])
+def test_a_group_holds_the_frames_its_budget_pays_for(gpu_ctx, tmp_path, disk, point):
+    import rtrace_b200 as rt
+    s = workloads.sphere_grid_scene()
+    light = {"position": [3, -3, 5], "color": "#FFFFFF", "intensity": 0.3}
+    s["lights"] = [dict(light, diameter=0.5) for _ in range(disk)] + [dict(light) for _ in range(point)]
+    scene = rt.Scene.from_json_file(workloads.write_scene(str(tmp_path), "s.json", s), gpu_ctx)
+    jobs = []
+    for k in range(6):
+        r = rt.Renderer(200, 150)
+        r.anti_aliasing_mode = rt.AntiAliasingMode.NoJitter
+        r.max_depth = 2
+        jobs.append(rt.Job(scene, r))
+    frame = 200 * 150 * (2 * 36 + 241 + 32 * (disk + point) + 57 * disk + 80)
+    saved = rt.batch_tuning(gpu_ctx)
+    try:
+        for frames in (2, 4, 5):
+            rt.batch_tuning(gpu_ctx, fuse_pixels=1 << 20, fuse_bytes=int((frames + 0.1) * frame))
+            rt.render_batch(jobs, lanes=2, ctx=gpu_ctx)
+            assert sum(j.renderer.last_stats.graph != 0 for j in jobs) == frames
+    finally:
+        rt.batch_tuning(gpu_ctx, lanes=saved["lanes"], fuse_pixels=saved["fuse_pixels"],
+                        fuse_bytes=saved["fuse_bytes"], blocks_per_sm=saved["blocks_per_sm"])
+    scene.close()
