@@ -1877,10 +1877,10 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
       for (int l = 0; l < levels; l++) hits += (uint64_t)nh[l];
       stats->reflection_rays = refl;
       stats->hits = hits;
-      // fallback hits recast their point lights and fb_dsamp rays per slot
-      // that falls back
+      // the fallback casts fb_dsamp rays per slot that falls back; point
+      // lights were answered before it
       stats->shadow_rays = (uint64_t)nh[0] * (uint64_t)K_0 + (hits - (uint64_t)nh[0]) * (uint64_t)K_full +
-                           (uint64_t)hfb[0] * (uint64_t)sc->n_point_lights + (uint64_t)hfb[1] * (uint64_t)fb_dsamp;
+                           (uint64_t)hfb[1] * (uint64_t)fb_dsamp;
       stats->fallback_hits = (uint64_t)hfb[0];
       stats->fallback_lights = (uint64_t)hfb[1];
       stats->shadow_rays_untraced = hstats[10];
