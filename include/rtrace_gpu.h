@@ -634,6 +634,10 @@ rt_status rt_debug_mesh_prep(rt_ctx* ctx, const rt_mesh_desc* mesh, uint32_t* mi
  * a wait between the stages of the queue levels that share a launch
  * (RT_ERR_DEVICE_WATCHDOG); 0: the default, 20 seconds. */
 rt_status rt_debug_set_barrier_limit(rt_ctx* ctx, int64_t ns);
+/* (Hit, light) pairs that the context's frames shade at once, at most 2^26;
+ * a queue level with more goes through the shading in chunks.  0: the
+ * default, 2^26. */
+rt_status rt_debug_set_chunk_pairs(rt_ctx* ctx, int64_t pairs);
 
 #ifdef __cplusplus
 }

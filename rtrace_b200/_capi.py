@@ -265,6 +265,7 @@ def lib():
         "rt_png_write": (ctypes.c_int, [ctypes.c_char_p, _vp, ctypes.c_uint32, ctypes.c_uint32]),
         "rt_debug_mesh_prep": (ctypes.c_int, [_vp, ctypes.POINTER(rt_mesh_desc), ctypes.POINTER(ctypes.c_uint32)]),
         "rt_debug_set_barrier_limit": (ctypes.c_int, [_vp, ctypes.c_int64]),
+        "rt_debug_set_chunk_pairs": (ctypes.c_int, [_vp, ctypes.c_int64]),
         "rt_debug_mesh_hit": (ctypes.c_int, [_vp, _vp, ctypes.c_int32, ctypes.c_int32, _vp, ctypes.c_int64,
                                              ctypes.c_double, ctypes.c_double, _vp]),
     }

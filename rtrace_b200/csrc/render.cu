@@ -113,6 +113,15 @@ struct FrameResult {
 // with the counts, hits, counters and error word copied one by one too).
 // Larger images gain nothing: the driver's own staging is as fast.
 constexpr size_t kPinImage = 1 << 20;
+// Shadow rays of one frame of a batch's fused group at most, and of the
+// learned pass (which holds a whole frame's hits).
+const long long kShadowCap = 1LL << 28;
+// (hit, light) pairs kept on the device at once: 32 bytes each, 57 more for
+// a disk light's (queue entries and three candidates), 6 GB at most; a
+// learned frame holds all of its hits' pairs, whose rays kShadowCap limits.
+// A 4K frame with 4 samples and two lights fits in one chunk per level:
+// chunks beyond a level's hits still cost their launches.
+const long long kPairCap = 1LL << 26;
 // A wait of k_levels' grid barrier gives up when nothing moved for this long.
 const long long kBarrierNs = 20000000000LL;
 
@@ -142,6 +151,7 @@ struct rt_ctx {
   int* d_err = nullptr;
   unsigned* d_bar = nullptr;  // k_levels' grid barrier
   long long barrier_ns = kBarrierNs;
+  long long pair_cap = kPairCap;
   int level_blocks = 0;       // blocks of k_levels that are resident together
   // learned soft shadows: network and its buffers (grown on demand)
   DenoiseNet net;
@@ -227,15 +237,6 @@ void drop_graphs(rt_ctx* ctx) {
 // replays instead of cycling through a too-small LRU.
 const size_t kMaxGraphs = 256;
 
-// Shadow rays of one frame of a batch's fused group at most, and of the
-// learned pass (which holds a whole frame's hits).
-const long long kShadowCap = 1LL << 28;
-// (hit, light) pairs kept on the device at once: 32 bytes each, 57 more for
-// a disk light's (queue entries and three candidates), 6 GB at most; a
-// learned frame holds all of its hits' pairs, whose rays kShadowCap limits.
-// A 4K frame with 4 samples and two lights fits in one chunk per level:
-// chunks beyond a level's hits still cost their launches.
-const long long kPairCap = 1LL << 26;
 // The first queue level of k_levels, and the frames it serves: at most this
 // many camera and shadow rays at the primary level, or objects that reflect.
 constexpr int kCoopLevel = 2;
@@ -1533,7 +1534,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
   const int n_lights = sc->n_point_lights + sc->n_disk_lights;
   if (learned && std::max(1LL, kShadowCap / K_0) < nprim)
     return fail(ctx, RT_ERR_INVALID_ARGUMENT, "too many primary samples for learned shadows in one pass");
-  const long long chunk = learned || !n_lights ? nprim : std::max(1LL, std::min(nprim, kPairCap / n_lights));
+  const long long chunk = learned || !n_lights ? nprim : std::max(1LL, std::min(nprim, ctx->pair_cap / n_lights));
   rt_status st = ensure_scratch(ctx, {nprim, levels, npix, chunk, chunk * n_lights, chunk * sc->n_disk_lights});
   if (st != RT_OK) return st;
   if (learned || want_aov) {
@@ -3021,6 +3022,12 @@ rt_status rt_debug_mesh_prep(rt_ctx* ctx, const rt_mesh_desc* md, uint32_t* mism
 rt_status rt_debug_set_barrier_limit(rt_ctx* ctx, int64_t ns) {
   if (!ctx || ns < 0) return fail(ctx, RT_ERR_INVALID_ARGUMENT, "bad argument");
   ctx->barrier_ns = ns ? ns : kBarrierNs;
+  return RT_OK;
+}
+
+rt_status rt_debug_set_chunk_pairs(rt_ctx* ctx, int64_t pairs) {
+  if (!ctx || pairs < 0 || pairs > kPairCap) return fail(ctx, RT_ERR_INVALID_ARGUMENT, "bad argument");
+  ctx->pair_cap = pairs ? pairs : kPairCap;
   return RT_OK;
 }
 
