@@ -1534,7 +1534,8 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
   const int n_lights = sc->n_point_lights + sc->n_disk_lights;
   if (learned && std::max(1LL, kShadowCap / K_0) < nprim)
     return fail(ctx, RT_ERR_INVALID_ARGUMENT, "too many primary samples for learned shadows in one pass");
-  const long long chunk = learned || !n_lights ? nprim : std::max(1LL, std::min(nprim, ctx->pair_cap / n_lights));
+  const long long chunk =
+      learned ? nprim : std::max(1LL, std::min(nprim, ctx->pair_cap / std::max(1, n_lights)));
   rt_status st = ensure_scratch(ctx, {nprim, levels, npix, chunk, chunk * n_lights, chunk * sc->n_disk_lights});
   if (st != RT_OK) return st;
   if (learned || want_aov) {

@@ -37,6 +37,23 @@ def test_chunks_match_one_pass(tmp_path, pairs):
     scene.close()
 
 
+# hits of a scene without lights, whose records are held all the same
+@pytest.mark.gpu
+def test_chunks_without_lights(tmp_path):
+    import rtrace_b200 as rt
+    ctx = rt.Context(0)
+    s = _scene(str(tmp_path), 1.0)
+    s["lights"] = []
+    scene = rt.Scene.from_json_file(workloads.write_scene(str(tmp_path), "s.json", s), ctx)
+    r = rt.Renderer(97, 55)
+    r.max_depth = 3
+    want, st = r.render(scene), r.last_stats
+    _chunk(ctx, 1000)
+    assert np.array_equal(r.render(scene), want)
+    assert r.last_stats.kernel_launches > st.kernel_launches
+    scene.close()
+
+
 # the visibility of a chunked level 0
 @pytest.mark.gpu
 def test_chunked_shadow_aov(tmp_path):
