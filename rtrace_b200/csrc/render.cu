@@ -201,6 +201,7 @@ rt_status fail(rt_ctx* ctx, rt_status s, const std::string& m) {
 }
 
 rt_status cuda_fail(rt_ctx* ctx, cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: a failed allocation is not the next launch's error
   rt_status s = (e == cudaErrorMemoryAllocation) ? RT_ERR_OUT_OF_MEMORY : RT_ERR_CUDA;
   return fail(ctx, s, std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -2844,11 +2845,10 @@ rt_status rt_denoiser_run(rt_ctx* ctx, const uint16_t* features, uint32_t planes
   if (st != RT_OK) return st;
   st = ensure_dn_arena(ctx, denoise_scratch_halves(ctx->net, (int)planes, (int)height, (int)width));
   if (st != RT_OK) return st;
-  // the scratch error word is shared with renders on this context
-  if (!ctx->d_err) {
-    st = ensure_scratch(ctx, {1, 1, 1, 1, 1, 1});
-    if (st != RT_OK) return st;
-  }
+  // the scratch error word is shared with renders on this context; there is
+  // none before the first and after one whose scratch did not fit
+  st = ensure_scratch(ctx, {1, 1, 1, 1, 0, 0});
+  if (st != RT_OK) return st;
   CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
   cudaError_t le = cudaSuccess;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));

@@ -76,3 +76,33 @@ def test_a_group_holds_the_frames_its_budget_pays_for(gpu_ctx, tmp_path, disk, p
         rt.batch_tuning(gpu_ctx, lanes=saved["lanes"], fuse_pixels=saved["fuse_pixels"],
                         fuse_bytes=saved["fuse_bytes"], blocks_per_sm=saved["blocks_per_sm"])
     scene.close()
+
+
+# a frame that no device holds gives back what the scratch held before it
+@pytest.mark.gpu
+def test_a_context_is_usable_after_a_frame_that_does_not_fit(tmp_path):
+    import torch
+    import rtrace_b200 as rt
+    from rtrace_b200 import _capi, denoiser
+    ctx = rt.Context(0)
+    ctx.load_denoiser(denoiser.pack(denoiser.random_layers(7)))
+    scene = rt.Scene.from_json_file(workloads.write_scene(str(tmp_path), "s.json", workloads.sphere_grid_scene()), ctx)
+    feat = torch.rand((1, 40, 60, 16), device="cuda").half()
+    torch.cuda.synchronize()
+
+    def net():
+        vis = torch.zeros((1, 2, 40, 60), device="cuda")
+        torch.cuda.synchronize()
+        L = _capi.lib()
+        assert L.rt_denoiser_run(ctx.handle, feat.data_ptr(), 1, 40, 60, vis.data_ptr(), None, None) == 0, \
+            L.rt_last_error(ctx.handle)
+        return vis
+    image, vis = rt.Renderer(64, 48).render(scene), net()
+    huge = rt.Renderer(30000, 30000)  # 1.8 billion rays: 900 GB
+    huge.anti_aliasing_mode, huge.samples = rt.AntiAliasingMode.Stochastic, 2
+    for _ in range(2):
+        with pytest.raises(rt.DeviceError, match="memory"):
+            huge.render(scene, device_ptr=feat.data_ptr())  # fails before anything is written
+        assert torch.equal(net(), vis)
+    assert np.array_equal(rt.Renderer(64, 48).render(scene), image)
+    scene.close()
