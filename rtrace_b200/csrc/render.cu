@@ -144,7 +144,8 @@ struct rt_ctx {
   std::vector<LevelBuf> h_levels;
   LevelBuf* d_levels = nullptr;
   FrameResult* d_res = nullptr;  // counts, hits, counters and the error word of a frame, as the host reads them back
-  char* pin_res = nullptr;       // pinned: a FrameResult, then a small image
+  FrameResult* pin_res = nullptr;  // pinned: *d_res
+  uint8_t* pin_img = nullptr;      // pinned: a small image; not for a batch's slots, which copy theirs out directly
   int* d_counts = nullptr;
   int* d_nhits = nullptr;
   unsigned long long* d_stats = nullptr;
@@ -333,7 +334,7 @@ rt_status ensure_scratch(rt_ctx* ctx, const ScratchDims& n) {
   ctx->d_stats = ctx->d_res->stats;
   ctx->d_err = &ctx->d_res->err;
   ctx->d_fbn = ctx->d_res->fbn;
-  if (!ctx->pin_res) CK(cudaMallocHost((void**)&ctx->pin_res, sizeof(FrameResult) + kPinImage));
+  if (!ctx->pin_res) CK(cudaMallocHost((void**)&ctx->pin_res, sizeof(FrameResult)));
   ctx->cap = d;
   return RT_OK;
 }
@@ -1637,6 +1638,8 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
     return RT_OK;
   }
 
+  const bool pinned = rgb_out && !on_device && (size_t)(3 * keep_pix) <= kPinImage;
+  if (pinned && !ctx->pin_img) CK(cudaMallocHost((void**)&ctx->pin_img, kPinImage));
   const bool count = (P->flags & RT_FLAG_COUNT_WORK) != 0;
   Launcher Lc{ctx, (P->flags & RT_FLAG_STAGE_TIMES) != 0};
   cudaStream_t s = ctx->stream;
@@ -1843,10 +1846,9 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
     if (es != RT_OK) return es;
   }
   CK(cudaEventRecord(ctx->ev1, s));
-  const bool pinned = rgb_out && !on_device && (size_t)(3 * keep_pix) <= kPinImage;
   if (rgb_out && !direct)
-    CK(cudaMemcpyAsync(pinned ? (uint8_t*)ctx->pin_res + sizeof(FrameResult) : rgb_out, d_rgb + 3 * keep_off,
-                       3 * keep_pix, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(pinned ? ctx->pin_img : rgb_out, d_rgb + 3 * keep_off, 3 * keep_pix,
+                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
   if (linear_out)
     CK(cudaMemcpyAsync(linear_out, d_linear + 3 * keep_off, 3 * keep_pix * sizeof(double), cudaMemcpyDeviceToHost,
                        s));
@@ -1854,8 +1856,8 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
   cudaError_t se = cudaStreamSynchronize(s);
   free_all(tmp);
   if (se != cudaSuccess) return cuda_fail(ctx, se, "render");
-  if (pinned) memcpy(rgb_out, ctx->pin_res + sizeof(FrameResult), 3 * keep_pix);
-  const FrameResult& res = *reinterpret_cast<const FrameResult*>(ctx->pin_res);
+  if (pinned) memcpy(rgb_out, ctx->pin_img, 3 * keep_pix);
+  const FrameResult& res = *ctx->pin_res;
   const int *counts = res.counts, *nh = res.nhits, herr = res.err;
   const unsigned long long* hstats = res.stats;
   const int hfb[2] = {fallback ? res.fbn[0] : 0, fallback ? res.fbn[1] : 0};
@@ -2083,7 +2085,7 @@ rt_status run_fused(rt_ctx* parent, rt_ctx* lane, rt_job* jobs, const std::vecto
   for (int j = 0; j < nj; j++) {
     const FramePlan& pl = plans[ok[j]];
     rt_job& J = jobs[idx[ok[j]]];
-    const FrameResult& back = *reinterpret_cast<const FrameResult*>(parent->slots[ok[j]]->pin_res);
+    const FrameResult& back = *parent->slots[ok[j]]->pin_res;
     const int herr = back.err;
     std::string msg;
     rt_status st = RT_OK;
@@ -2174,7 +2176,9 @@ void rt_ctx_destroy(rt_ctx* ctx) {
   if (ctx->pin) cudaFreeHost(ctx->pin);
   ctx->pin = nullptr;
   if (ctx->pin_res) cudaFreeHost(ctx->pin_res);
+  if (ctx->pin_img) cudaFreeHost(ctx->pin_img);
   ctx->pin_res = nullptr;
+  ctx->pin_img = nullptr;
   drop_graphs(ctx);
   free_all(ctx->scratch);
   free_all(ctx->dn_scratch);

@@ -106,3 +106,27 @@ def test_a_context_is_usable_after_a_frame_that_does_not_fit(tmp_path):
         assert torch.equal(net(), vis)
     assert np.array_equal(rt.Renderer(64, 48).render(scene), image)
     scene.close()
+
+
+# pinned host memory of a group's frames: their results, a kilobyte each, and no
+# image buffer that no frame of a group uses
+@pytest.mark.gpu
+def test_a_group_of_many_frames_pins_little_host_memory(tmp_path):
+    import rtrace_b200 as rt
+
+    def pinned_mb():
+        return next(int(line.split()[1]) for line in open("/proc/self/status") if line.startswith("RssShmem")) / 1024
+    ctx = rt.Context(0)
+    scene = rt.Scene.from_json_file(workloads.write_scene(str(tmp_path), "s.json", workloads.sphere_grid_scene()), ctx)
+    jobs = []
+    for _ in range(128):
+        r = rt.Renderer(16, 12)
+        r.max_depth = 2
+        jobs.append(rt.Job(scene, r))
+    want = jobs[0].renderer.render(scene)
+    rt.batch_tuning(ctx, fuse_pixels=1 << 20)
+    before = pinned_mb()
+    images, _ = rt.render_batch(jobs, lanes=1, ctx=ctx)
+    assert pinned_mb() - before < 32
+    assert all(j.renderer.last_stats.graph != 0 for j in jobs) and all(np.array_equal(i, want) for i in images)
+    scene.close()
