@@ -69,3 +69,32 @@ def test_a_wait_that_runs_out_is_an_error(tmp_path):
         _limit(ctx, 0)
         assert np.array_equal(r.render(scene), want)
     scene.close()
+
+
+# contexts on threads of their own, whose launches each want the whole device
+@pytest.mark.gpu
+def test_contexts_on_threads_share_the_device(tmp_path):
+    import threading
+    import rtrace_b200 as rt
+    s = _scene()
+    s["objects"] = s["objects"][:40]
+    path = workloads.write_scene(str(tmp_path), "s.json", s)
+    r = rt.Renderer(160, 120)
+    r.max_depth = 6
+    want = r.render(rt.Scene.from_json_file(path, rt.Context(0)))
+    right = []
+
+    def work():
+        ctx = rt.Context(0)
+        scene = rt.Scene.from_json_file(path, ctx)
+        mine = rt.Renderer(160, 120)
+        mine.max_depth = 6
+        for _ in range(25):
+            right.append(np.array_equal(mine.render(scene), want))
+        scene.close()
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(right) == 100 and all(right)
