@@ -430,7 +430,6 @@ __device__ __forceinline__ bool tri_first_visit(const DMesh& M, const RayC& r, i
 // The exact reference k-d walk (MeshObject::hit with KdTree::traverse,
 // src/ray.rs:614-649, src/mesh.rs:399-465) with exact subtree culling by
 // node bounds and closest-t pruning.  Returns the winning triangle index.
-template <bool ANY>
 __device__ bool mesh_kd_walk(const DMesh& M, const RayC& r, double tmin, double& closest, int& best_tri, int* err,
                              Work* w) {
   if (M.n_nodes == 0) return false;
@@ -457,7 +456,6 @@ __device__ bool mesh_kd_walk(const DMesh& M, const RayC& r, double tmin, double&
             closest = t;
             best_tri = tri;
             found = true;
-            if (ANY) return true;
           }
         }
       } else {
@@ -737,7 +735,7 @@ __device__ bool mesh_closest(const DMesh& M, V3 o, V3 d, double tmin, double& cl
   }
   // The reference does not test the nearest triangle (or too many tie):
   // answer with the reference's own walk.
-  return mesh_kd_walk<false>(M, r, tmin, closest, best_tri, err, w);
+  return mesh_kd_walk(M, r, tmin, closest, best_tri, err, w);
 }
 
 // A run of spheres: minimal accepted root, ties to the latest sphere.  On

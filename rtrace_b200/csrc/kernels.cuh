@@ -1672,7 +1672,7 @@ __global__ void __launch_bounds__(128) k_debug_mesh(DMesh M, int use_kd, int mod
     }
     bool hit = valid && (mode == 0 ? mesh_closest(M, o, d, tmin, closest, best, use_kd != 0, err, nullptr)
                                    : (mesh_bounds(M, r, tmin, closest) &&
-                                      mesh_kd_walk<false>(M, r, tmin, closest, best, err, nullptr)));
+                                      mesh_kd_walk(M, r, tmin, closest, best, err, nullptr)));
     if (!valid) continue;
     for (int k = 0; k < 8; k++) oo[k] = 0.0;
     if (hit) {
