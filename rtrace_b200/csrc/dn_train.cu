@@ -29,6 +29,12 @@
 #include "denoise.hpp"
 
 namespace rtb {
+// k_wgrad_tc's bias gradient of one launch, over its CTAs; zero between launches.
+struct WgBias {
+  double sum[64];
+  unsigned done;
+};
+
 namespace {
 
 constexpr float kLossScale = 256.0f;  // FP16 gradients: scaled sums, divided out in the Adam step
@@ -77,23 +83,40 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr));
 }
 
+__device__ __forceinline__ void h8_to_f(const uint4& v, float (&f)[8]) {
+  const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float2 t = __half22float2(h[k]);
+    f[2 * k] = t.x;
+    f[2 * k + 1] = t.y;
+  }
+}
+__device__ __forceinline__ uint4 f_to_h8(const float (&f)[8]) {
+  uint4 v;
+  __half2* h = reinterpret_cast<__half2*>(&v);
+#pragma unroll
+  for (int k = 0; k < 4; k++) h[k] = __floats2half2_rn(f[2 * k], f[2 * k + 1]);
+  return v;
+}
+
 constexpr int WG_THREADS = 128;
 constexpr int WG_TILE = 128;  // pixels of one row per step (the GEMM's K per step)
 
-// Shared memory of one k_wgrad_tc CTA: `stages` stages of three input rows, a
-// row of ones and the dZ run.  An M block of the GEMM is 128 / CIN of a
-// stage's rows from its first one on; with 16 channels it reads past the
-// ones into whatever follows: accumulator rows nobody reads.
+// Shared memory of one k_wgrad_tc CTA: `stages` stages of three input rows
+// and the dZ run.  An M block of the GEMM is 128 / CIN of a stage's rows from
+// its first one on; beyond the third it reads whatever follows: accumulator
+// rows nobody reads.
 template <int CIN, int COUT>
 struct WgSmem {
   static constexpr int PER = 128 / CIN;             // staged rows per M block
-  static constexpr int MB = (4 + PER - 1) / PER;    // M blocks
+  static constexpr int MB = (3 + PER - 1) / PER;    // M blocks
   static constexpr int COLS = 3 * MB * COUT;        // accumulators: 3 kx x MB x COUT columns
   static constexpr int TMEM = COLS <= 32 ? 32 : COLS <= 64 ? 64 : COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
-  static constexpr int TAIL = 256;
+  static constexpr int TAIL = 256 + 2 * COUT * 8;   // barriers and flags, the bias warps' sums
   static int px(int dil, int kxs) { return kxs == 3 ? WG_TILE + 2 * dil : WG_TILE; }
   static __host__ __device__ int row(int px) { return (px * CIN * 2 + 1023) / 1024 * 1024; }
-  static __host__ __device__ int stage(int row) { return 4 * row + WG_TILE * COUT * 2; }
+  static __host__ __device__ int stage(int row) { return 3 * row + WG_TILE * COUT * 2; }
   static __host__ __device__ int pad(int row) {
     const int over = PER * MB * row - stage(row);
     return over > 0 ? over : 0;
@@ -119,15 +142,21 @@ __device__ __forceinline__ void tma_row(uint32_t dst, const CUtensorMap* map, in
 // the same K.  The channels are the contiguous dimension of both tensors, so
 // both operands are MN-major and TMA stages them as they lie, a row of all
 // channels per pixel; the shift by kx * dil pixels is an offset of the
-// descriptor's start.  A's fourth row holds ones: its result is the bias
-// gradient.
+// descriptor's start.
 //
 // Warp 0 loads the stages (one 128-pixel run of one row per step, zero-filled
 // beyond the image), warp 1 issues the MMAs into accumulators that stay in
 // tensor memory for all of the CTA's steps; at the end every thread adds its
 // accumulator rows into dW with FP32 atomics.  Waits are bounded; one that
-// runs out sets err, both roles leave their loops and wait (bounded) for
+// runs out sets err, all roles leave their loops and wait (bounded) for
 // what they have in flight before the tensor memory is released.
+//
+// Warps 2 and 3 sum the staged dZ runs for the bias gradient: at most 16
+// pixels in FP32, the runs in double, the CTAs by double atomics, and the last
+// CTA rounds the total into db.  The tensor pipe, as a row of ones under the
+// inputs, truncated instead of rounding: dZ of one sign, 16 x 256 x 256 pixels,
+// 32 channels: 2.8e-6 of the sum off, 2.5e-8 here (1.4e-7 in FP32 by threads
+// of every 128-pixel run).
 //
 // kxs = 1: dilations above 64, whose halo exceeds a TMA box; a step then
 // loads the rows for one kx.
@@ -141,14 +170,14 @@ template <int CIN, int COUT>
 __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__ CUtensorMap xmap,
                                                          const __grid_constant__ CUtensorMap zmap, int planes, int H,
                                                          int W, int dil, int kxs, int stages, float* __restrict__ dW,
-                                                         float* __restrict__ db, int* err) {
+                                                         float* __restrict__ db, WgBias* bias, int* err) {
   using SM = WgSmem<CIN, COUT>;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;
   const uint32_t s0 = raw + pad;
   const int px = kxs == 3 ? WG_TILE + 2 * dil : WG_TILE;
-  const int ROW = SM::row(px), STAGE = SM::stage(ROW), ZOFF = 4 * ROW;
+  const int ROW = SM::row(px), STAGE = SM::stage(ROW), ZOFF = 3 * ROW;
   unsigned char* tail = smem_raw + pad + stages * STAGE + SM::pad(ROW);
   const uint32_t bar0 = smem_u32(tail);  // full[8], empty[8], done
   auto full_bar = [&](int k) { return bar0 + 8u * k; };
@@ -157,16 +186,14 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__
   uint32_t* tslot = reinterpret_cast<uint32_t*>(tail + 8 * 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8 * 17 + 4);
   int* s_used = reinterpret_cast<int*>(tail + 8 * 17 + 8);  // kx whose accumulators hold a sum
+  int* s_last = reinterpret_cast<int*>(tail + 8 * 17 + 12);
+  double* s_db = reinterpret_cast<double*>(tail + 256);  // [2][COUT]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // the ones of every stage
-  for (int i = tid; i < stages * ROW / 4; i += WG_THREADS) {
-    const int st = i / (ROW / 4), o = i % (ROW / 4);
-    reinterpret_cast<uint32_t*>(smem_raw + pad + st * STAGE + 3 * ROW)[o] = 0x3C003C00u;
-  }
   if (tid == 0) {
     for (int k = 0; k < stages; k++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full_bar(k)) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty_bar(k)) : "memory");
+      // the step's MMAs and the two bias warps
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 3;" ::"r"(empty_bar(k)) : "memory");
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(done_bar) : "memory");
     *abort_flag = 0;
@@ -265,6 +292,40 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__
                    : "memory");
       if (!mbar_wait(done_bar, 0)) fail();
     }
+  } else {
+    constexpr int CH = COUT / 8, STEP = 64 / CH;  // 8-channel groups; pixels apart of a thread's
+    const int c = lane % CH, p0 = (tid - 64) / CH;
+    double sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    long long n = 0;
+    for (long long st = blockIdx.x; st < nsteps; st += gridDim.x, n++) {
+      const int k = (int)(n % stages);
+      const bool ok = !*abort_flag && mbar_wait(full_bar(k), (uint32_t)((n / stages) & 1));
+      if (!__all_sync(0xffffffffu, ok)) {
+        fail();
+        break;
+      }
+      if (st % sub == 0) {  // a run's steps hold the same dZ
+        const unsigned char* z = smem_raw + pad + k * STAGE + ZOFF;
+        float run[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < WG_TILE / STEP; i++) {
+          const uint32_t o = (uint32_t)((p0 + i * STEP) * COUT * 2 + c * 16);
+          float f[8];
+          h8_to_f(*reinterpret_cast<const uint4*>(z + (o ^ ((o >> 3) & (COUT * 2 - 16)))), f);  // as TMA swizzles it
+#pragma unroll
+          for (int e = 0; e < 8; e++) run[e] += f[e];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) sum[e] += run[e];
+      }
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar(k)) : "memory");
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      for (int off = 16; off >= CH; off >>= 1) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], off);
+      if (lane < CH) s_db[(warp - 2) * COUT + 8 * lane + e] = sum[e];
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -275,7 +336,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__
     for (int kx = 0; kx < 3; kx++) {
       if (!((used >> kx) & 1)) continue;
       for (int m = 0; m < SM::MB; m++) {
-        const int ky = m * SM::PER + tid / CIN, ci = tid % CIN;  // ky = 3: the ones
+        const int ky = m * SM::PER + tid / CIN, ci = tid % CIN;
 #pragma unroll
         for (int c0 = 0; c0 < COUT; c0 += 16) {
           uint32_t v[16];
@@ -285,16 +346,27 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__
 #pragma unroll
             for (int k = 0; k < 16; k++)
               atomicAdd(&dW[((size_t)(c0 + k) * 9 + 3 * ky + kx) * CIN + ci], __uint_as_float(v[k]));
-          } else if (ky == 3 && kx == 0 && ci == 0) {
-#pragma unroll
-            for (int k = 0; k < 16; k++) atomicAdd(&db[c0 + k], __uint_as_float(v[k]));
           }
         }
       }
     }
+    if (tid < COUT) {
+      atomicAdd(&bias->sum[tid], s_db[tid] + s_db[COUT + tid]);
+      __threadfence();
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (tid == 0) *s_last = atomicAdd(&bias->done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (*s_last) {
+    __threadfence();
+    if (tid < COUT) {
+      db[tid] += (float)*(volatile double*)&bias->sum[tid];
+      bias->sum[tid] = 0.0;
+    }
+    if (tid == 0) bias->done = 0;
+  }
   if (warp == 2) {
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -304,7 +376,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__
 
 template <int CIN, int COUT>
 cudaError_t launch_wgrad(const __half* X, const __half* dZ, int planes, int H, int W, int dil, float* dW, float* db,
-                         int* err, cudaStream_t s, int num_sms) {
+                         WgBias* bias, int* err, cudaStream_t s, int num_sms) {
   using SM = WgSmem<CIN, COUT>;
   const int kxs = dil <= 64 ? 3 : 1;
   const int row = SM::row(SM::px(dil, kxs));
@@ -334,28 +406,11 @@ cudaError_t launch_wgrad(const __half* X, const __half* dZ, int planes, int H, i
   if ((e = make_row_map(&zmap, dZ, planes, H, W, COUT, WG_TILE)) != cudaSuccess) return e;
   const long long nsteps = (long long)planes * H * ((W + WG_TILE - 1) / WG_TILE) * (kxs == 3 ? 1 : 3);
   const int grid = (int)std::max<long long>(1, std::min<long long>(nsteps, (long long)ctas * num_sms));
-  k_wgrad_tc<CIN, COUT><<<grid, WG_THREADS, smem, s>>>(xmap, zmap, planes, H, W, dil, kxs, stages, dW, db, err);
+  k_wgrad_tc<CIN, COUT><<<grid, WG_THREADS, smem, s>>>(xmap, zmap, planes, H, W, dil, kxs, stages, dW, db, bias, err);
   return cudaGetLastError();
 }
 
 // ---- elementwise kernels of the backward pass (8 FP16 channels a thread)
-__device__ __forceinline__ void h8_to_f(const uint4& v, float (&f)[8]) {
-  const __half2* h = reinterpret_cast<const __half2*>(&v);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const float2 t = __half22float2(h[k]);
-    f[2 * k] = t.x;
-    f[2 * k + 1] = t.y;
-  }
-}
-__device__ __forceinline__ uint4 f_to_h8(const float (&f)[8]) {
-  uint4 v;
-  __half2* h = reinterpret_cast<__half2*>(&v);
-#pragma unroll
-  for (int k = 0; k < 4; k++) h[k] = __floats2half2_rn(f[2 * k], f[2 * k + 1]);
-  return v;
-}
-
 #define RTB_GRID_STRIDE(t, n) \
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (n); t += (long long)gridDim.x * blockDim.x)
 
@@ -573,9 +628,9 @@ int level_dim(int n, int level) { return (n + (1 << level) - 1) >> level; }
 }  // namespace
 
 cudaError_t wgrad_launch(int cin, int cout, const __half* X, const __half* dZ, int planes, int H, int W, int dil,
-                         float* dW, float* db, int* err, cudaStream_t s, int num_sms) {
+                         float* dW, float* db, WgBias* bias, int* err, cudaStream_t s, int num_sms) {
 #define RTB_WG(CI, CO) \
-  if (cin == CI && cout == CO) return launch_wgrad<CI, CO>(X, dZ, planes, H, W, dil, dW, db, err, s, num_sms);
+  if (cin == CI && cout == CO) return launch_wgrad<CI, CO>(X, dZ, planes, H, W, dil, dW, db, bias, err, s, num_sms);
   RTB_WG(16, 16)
   RTB_WG(16, 32)
   RTB_WG(32, 16)
@@ -604,6 +659,7 @@ struct rt_dn_trainer {
   float *master = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *acc = nullptr, *zeros = nullptr;
   double* part = nullptr;    // k_loss: partial sums
   unsigned* done = nullptr;  // and its block count
+  WgBias* bias = nullptr;    // k_wgrad_tc's
   long long n_params = 0;
   __half *arena = nullptr, *gbuf = nullptr, *dz = nullptr, *tmp = nullptr;
   std::vector<size_t> act_off, g_off;  // per buffer (1..n): offsets in arena / gbuf (halves)
@@ -704,12 +760,14 @@ rt_status rt_dn_train_create(rt_ctx* ctx, const void* blob, size_t bytes, uint32
   };
   if (talloc(t, &t->master, host.size()) || talloc(t, &t->m1, host.size()) || talloc(t, &t->m2, host.size()) ||
       talloc(t, &t->grad, host.size()) || talloc(t, &t->acc, 4) || talloc(t, &t->zeros, 64) ||
-      talloc(t, &t->part, 3 * 16 * (size_t)ctx_num_sms(ctx)) || talloc(t, &t->done, 1) || talloc(t, &t->err, 1))
+      talloc(t, &t->part, 3 * 16 * (size_t)ctx_num_sms(ctx)) || talloc(t, &t->done, 1) || talloc(t, &t->bias, 1) ||
+      talloc(t, &t->err, 1))
     return bad("optimizer");
   cudaStream_t s = ctx_stream(ctx);
   if (cudaMemcpyAsync(t->master, host.data(), host.size() * 4, cudaMemcpyHostToDevice, s) ||
       cudaMemsetAsync(t->m1, 0, host.size() * 4, s) || cudaMemsetAsync(t->m2, 0, host.size() * 4, s) ||
-      cudaMemsetAsync(t->zeros, 0, 64 * 4, s) || cudaMemsetAsync(t->done, 0, 4, s))
+      cudaMemsetAsync(t->zeros, 0, 64 * 4, s) || cudaMemsetAsync(t->done, 0, 4, s) ||
+      cudaMemsetAsync(t->bias, 0, sizeof(WgBias), s))
     return bad("upload");
   for (size_t i = 0; i < t->net.ops.size(); i++) {
     DnOp& o = t->net.ops[i];
@@ -817,7 +875,7 @@ rt_status train_grads(rt_dn_trainer* t, const __half* feat, const __half* target
       const int c = t->conv_of_op[ii];
       float* dW = t->grad + t->woff[c];
       float* db = dW + (size_t)o.cout * 9 * o.cin;
-      if (!CKE(wgrad_launch(o.cin, o.cout, act[o.src], dz, P, h, w, o.dil, dW, db, t->err, s, nsm), "wgrad"))
+      if (!CKE(wgrad_launch(o.cin, o.cout, act[o.src], dz, P, h, w, o.dil, dW, db, t->bias, t->err, s, nsm), "wgrad"))
         return RT_ERR_CUDA;
       (*launches)++;
       if (o.src > 0) {
@@ -976,18 +1034,20 @@ rt_status rt_debug_conv_wgrad(rt_ctx* ctx, const uint16_t* x, const uint16_t* dz
   if (!ctx || !x || !dz || !dw || !db) return ctx_fail(ctx, RT_ERR_INVALID_ARGUMENT, "null argument");
   cudaSetDevice(ctx_device(ctx));
   cudaStream_t s = ctx_stream(ctx);
-  int* err = nullptr;
-  if (cudaMalloc((void**)&err, 4) != cudaSuccess) return ctx_fail(ctx, RT_ERR_OUT_OF_MEMORY, "cudaMalloc");
-  cudaMemsetAsync(err, 0, 4, s);
+  WgBias* bias = nullptr;  // and the error word behind it
+  if (cudaMalloc((void**)&bias, sizeof(WgBias) + 4) != cudaSuccess)
+    return ctx_fail(ctx, RT_ERR_OUT_OF_MEMORY, "cudaMalloc");
+  cudaMemsetAsync(bias, 0, sizeof(WgBias) + 4, s);
+  int* err = reinterpret_cast<int*>(bias + 1);
   cudaError_t e = wgrad_launch((int)cin, (int)cout, reinterpret_cast<const __half*>(x),
                                reinterpret_cast<const __half*>(dz), (int)planes, (int)height, (int)width, (int)dil, dw,
-                               db, err, s, ctx_num_sms(ctx));
+                               db, bias, err, s, ctx_num_sms(ctx));
   int herr = 0;
   if (e == cudaSuccess) {
     cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);
   }
-  cudaFree(err);
+  cudaFree(bias);
   if (e != cudaSuccess) return ctx_fail(ctx, RT_ERR_CUDA, std::string("wgrad: ") + cudaGetErrorString(e));
   if (herr & DN_ERR_WAIT) return ctx_fail(ctx, RT_ERR_DEVICE_WATCHDOG, "wgrad: a tensor-core wait timed out");
   return RT_OK;
