@@ -51,6 +51,7 @@ struct DCube {
   double w2l[12];  // rows 0..2 of the world-to-local matrix
   double l2w[12];  // rows 0..2 of the local-to-world matrix
   double ntr[9];   // inverse-transpose of w2l's rotation part
+  double bound[4];  // a world sphere around it, of infinite radius where none is known
   int identity;
   int pad;
 };
@@ -968,6 +969,23 @@ __device__ __forceinline__ bool cone_sphere(const Cone& k, const double* s, bool
   return true;
 }
 
+// Whether the cone can meet the cube, by its bounding sphere.  Cube::hit
+// measures t in the cube's own frame, so a scaled cube may block from beyond
+// the light: its sphere is tested against the cone without an end.
+__device__ __forceinline__ bool cone_cube(const Cone& k, const DCube& C) {
+  const V3 v = ld3(C.bound) - k.o;
+  const double a = dot(v, k.c), vv = dot(v, v);
+  const double r = C.bound[3] * (1.0 + 1e-5) + 1e-5 * sum_abs(v) + 1e-8 * sum_abs(k.o);
+  if (!(vv < 1e200 && r < 1e100) || vv <= r * r) return true;
+  if (C.identity && a > k.D + r) return false;
+  if (v.x * k.h[0] + v.y * k.h[1] + v.z * k.h[2] < -r) return false;
+  const double p2 = fmax(vv - a * a, 0.0);
+  // behind the apex, whose distance then is the cone's
+  if (a < 0.0 && a * a * k.ca * k.ca > p2 * k.sa * k.sa * (1.0 + 1e-5)) return false;
+  const double reach = k.T * a + r / k.ca;
+  return !(reach < 0.0 || p2 > reach * reach);
+}
+
 // Whether the cone can cross the plane through q with normal n (any
 // length; `size`: the magnitude of the terms its distances are sums of).
 __device__ __forceinline__ bool cone_plane(const Cone& k, V3 q, V3 n, double size) {
@@ -1024,8 +1042,9 @@ __device__ __forceinline__ int shaft_collect(const DScene& S, const Cone& k, int
         const double* p = S.pln + 12 * (size_t)ob.y;
         const V3 q = mk(p[0], p[1], p[2]), pn = mk(p[3], p[4], p[5]);
         if (!cone_plane(k, q, pn, sum_abs(pn) * (sum_abs(k.o) + sum_abs(q) + k.D))) continue;
+      } else if (!cone_cube(k, S.cub[ob.y])) {
+        continue;
       }
-      // a cube's own test measures t in its local frame: always a candidate
       if (n == RTB_CAND) return CONE_MANY;
       out[n * stride] = make_int2(i, 0);
       n++;

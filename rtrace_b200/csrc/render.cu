@@ -1119,6 +1119,30 @@ const int kMinSphereRun = 8;
 // Uploads a scene description.  preps, when given, holds one prepared mesh
 // per d->meshes entry (kept by a host scene); missing entries are prepared
 // here and stored into it.
+// The world sphere around a cube whose points x satisfy |a (x - c)| <= half on
+// every axis, ai the inverse of a.  Infinite where the map is too far from a
+// rotation for the cones' margins, or the cube is no box.
+void cube_bound(DCube& C, const double a[3][3], const double ai[3][3], bool invertible) {
+  double na = 0.0, nai = 0.0, r2 = 0.0;
+  for (int r = 0; r < 3; r++)
+    for (int c = 0; c < 3; c++) {
+      na += a[r][c] * a[r][c];
+      nai += ai[r][c] * ai[r][c];
+    }
+  for (int corner = 0; corner < 4; corner++) {
+    double d2 = 0.0;
+    for (int r = 0; r < 3; r++) {
+      const double x = ai[r][0] * C.half[0] + (corner & 1 ? -1 : 1) * ai[r][1] * C.half[1] +
+                       (corner & 2 ? -1 : 1) * ai[r][2] * C.half[2];
+      d2 += x * x;
+    }
+    r2 = std::max(r2, d2);
+  }
+  const bool box = C.half[0] >= 0.0 && C.half[1] >= 0.0 && C.half[2] >= 0.0;
+  for (int k = 0; k < 3; k++) C.bound[k] = C.c[k];
+  C.bound[3] = invertible && box && na * nai < 1e12 && r2 < 1e200 ? std::sqrt(r2) : INFINITY;
+}
+
 rt_status do_upload(rt_ctx* ctx, const rt_scene_desc* d, rt_scene** out,
                     std::vector<std::shared_ptr<MeshPrep>>* preps = nullptr) {
   if (!d) return fail(ctx, RT_ERR_INVALID_ARGUMENT, "null scene description");
@@ -1220,7 +1244,9 @@ rt_status do_upload(rt_ctx* ctx, const rt_scene_desc* d, rt_scene** out,
       double a[3][3], ri[3][3];
       for (int r = 0; r < 3; r++)
         for (int c = 0; c < 3; c++) a[r][c] = inv[4 * r + c];
-      if (!inverse3(a, ri))
+      const bool invertible = inverse3(a, ri);
+      cube_bound(C, a, ri, invertible);
+      if (!invertible)
         for (int r = 0; r < 3; r++)
           for (int c = 0; c < 3; c++) ri[r][c] = r == c ? 1.0 : 0.0;
       for (int r = 0; r < 3; r++)
