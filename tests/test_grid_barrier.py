@@ -11,12 +11,13 @@ MAT = workloads._mat
 
 def _scene():
     """Two facing mirrors, so that every level has all of its rays, and 1,000
-    cubes that every shadow ray tests one by one."""
+    cubes that every shadow ray tests one by one: too flat for the light cones
+    to leave them out."""
     objs = [{"kind": "plane", "point": [0, 0, z], "normal": [0, 0, n], "material": MAT("#909090", reflectivity=0.6)}
             for z, n in ((-1, 1), (1, -1))]
     for k in range(1000):
         objs.append({"kind": "cube", "center": [-50 - k % 10, k // 100, (k // 10) % 10 * 0.1], "size": [0.05, 0.05, 0.05],
-                     "material": MAT("#4040C0")})
+                     "transform": ["scale(1, 1, 0.0000001)"], "material": MAT("#4040C0")})
     return {"camera": {"kind": "perspective", "position": [0, -8, 0], "target": [0, 0, 0.3], "up": [0, 0, 1], "fov": 50,
                        "width": 16, "height": 9},
             "objects": objs,
