@@ -69,6 +69,7 @@ struct DFrame {
   // Shadow rays per disk light at the current level, set by the host (the
   // reference casts 16), and log2 of the lanes that share a light in k_part.
   int dsamp, lanes_log2;
+  int walk;  // k_walk runs at this level, where walked pairs are many
   // Learned soft shadows (extension): at level 0 each disk light gets one
   // ray, and its visibility comes from the denoiser's vhat
   // ([plane][slot][H][W], plane = sample index within the pixel).
@@ -685,7 +686,10 @@ __global__ void __launch_bounds__(128, 8) k_shaft_multi(const DFrame* __restrict
 // g: a lane per sample (at most 32) makes the most of few pairs; a pair per
 // lane (g = 1) saves the work that a group's lanes repeat (the hit, the
 // light's frame, the blocks beyond those the samples need), so g halves
-// while the pairs still fill the chip.  The walked pairs keep theirs.
+// while the pairs still fill the chip.  Walked pairs keep more of them, as a
+// pair's rays take similar walks: g halves from 2^22 lanes on (2^18 to 2^21,
+// 1280x720: 8 to 37% more on a low light over terrain, up to 9% less under
+// lights wider than their distance; never: 14% more there).
 //
 // Bound by instruction issue and by the code's own size: at 900 instructions
 // per sample and warp the loop outgrows the instruction cache.  1,000-sphere
@@ -702,6 +706,8 @@ __global__ void __launch_bounds__(128, 8) k_shaft_multi(const DFrame* __restrict
 // leave the normal range, draw serially (StdRng) on the group's first lane.
 #define PART_RING 8         // ring entries per lane; a round adds at most 4
 #define PART_FILL (1 << 17)  // lanes that fill the chip
+#define WALK_FILL (1 << 22)  // and lanes that share out many walks
+#define WALK_MANY (1 << 18)  // walked pairs that k_walk takes
 struct PartShared {
   double2 off[4][32 * PART_RING];
   double term[4][3][32];
@@ -710,8 +716,7 @@ struct PartShared {
 template <int KIND>
 __device__ __forceinline__ int part_lanes(const DFrame& F, int n) {
   int lg = F.lanes_log2;
-  if (KIND != PART_WALK)
-    while (lg > 0 && ((long long)n << (lg - 1)) >= PART_FILL) lg--;
+  while (lg > 0 && ((long long)n << (lg - 1)) >= (KIND == PART_WALK ? WALK_FILL : PART_FILL)) lg--;
   return lg;
 }
 template <int KIND>
@@ -930,13 +935,27 @@ __device__ __forceinline__ void part_all(const DFrame& F, int level, long long c
   // the warp's first task of a class that follows `tasks` others
   auto next = [&](int tasks) { w0 = (w0 + nw - tasks % nw) % nw; };
   auto mine = [&](int k) { return part < 0 || part == k ? w0 : none; };
-  part_body<PART_WALK, COUNT>(F, level, c0, sm, mine(0), nw, steps);
+  part_body<PART_WALK, COUNT>(F, level, c0, sm, F.walk && F.pair.n[PART_WALK] >= WALK_MANY ? none : mine(0), nw, steps);
   if (part < 0) next(part_tasks<PART_WALK>(F));
   part_body<PART_LIST, COUNT>(F, level, c0, sm, mine(1), nw, steps);
   if (part < 0) next(part_tasks<PART_LIST>(F));
   part_body<PART_LIT2, COUNT>(F, level, c0, sm, lit ? mine(2) : none, nw, steps);
   if (part < 0) next(part_tasks<PART_LIT2>(F));
   part_body<PART_LIT, COUNT>(F, level, c0, sm, lit ? mine(3) : none, nw, steps);
+}
+// The walked pairs of a level where they are many, before k_part: walks wait
+// for their node loads, and without the other classes' code 6 blocks of 128
+// share an SM (80 registers; 8 blocks within 4%, 10 up to 60% slower).
+// 1280x720: icosphere under a light as wide as its distance 7.2 -> 6.2 ms, low
+// light over terrain 9.7 -> 8.5, 1,000 spheres under lights of diameter 16 11.0
+// -> 10.2.  Fewer than 2^18 pairs (2^20: the first two as without) fill the
+// chip beside the other queues' blocks, and frames with few walks pay 5 us for
+// a launch that returns.
+template <bool COUNT>
+__global__ void __launch_bounds__(128, 6) k_walk(const __grid_constant__ DFrame F, int level, long long c0) {
+  __shared__ PartShared sm;
+  if (F.pair.n[PART_WALK] < WALK_MANY) return;
+  part_body<PART_WALK, COUNT>(F, level, c0, sm, 4LL * blockIdx.x + (threadIdx.x >> 5), 4LL * gridDim.x, nullptr);
 }
 template <bool COUNT>
 __global__ void __launch_bounds__(128, 4) k_part(const __grid_constant__ DFrame F, int level, long long c0) {

@@ -1682,6 +1682,12 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
   };
   auto launch_part = [&](const DFrame& Fp, int level, long long c0) {
     const int grid = 4 * blocks((chunk * sc->n_disk_lights) << Fp.lanes_log2, 128, 32);
+    if (Fp.walk && !Fp.fb_mode) {
+      const int g = blocks((chunk * sc->n_disk_lights) << 2, 128, 64);
+      if (count) k_walk<true><<<g, 128, 0, s>>>(Fp, level, c0);
+      else k_walk<false><<<g, 128, 0, s>>>(Fp, level, c0);
+      Lc.after(RT_STAGE_SHADOW);
+    }
     if (count) k_part<true><<<grid, 128, 0, s>>>(Fp, level, c0);
     else k_part<false><<<grid, 128, 0, s>>>(Fp, level, c0);
     Lc.after(RT_STAGE_SHADOW);
@@ -1722,6 +1728,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
         // rays per disk light at this level
         F.dsamp = (l == 0 && learned) ? lrays : dsamp;
         F.lanes_log2 = pair_lanes_log2(F.dsamp);
+        F.walk = l <= 1 && chunk * sc->n_disk_lights >= WALK_MANY;  // deeper levels seldom have as many
         const bool feat = l == 0 && F.feat_on;
         const long long nchunks = (nprim + chunk - 1) / chunk;
         // The walks' grids hold many more blocks than stay resident (64 per
@@ -1773,6 +1780,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
             Lc.after(RT_STAGE_DENOISE);
             DFrame Fb = F;
             Fb.fb_mode = 1;
+            Fb.walk = 0;
             Fb.dsamp = fb_dsamp;
             Fb.lanes_log2 = pair_lanes_log2(fb_dsamp);
             launch_part(Fb, 0, 0);
@@ -1784,6 +1792,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
       if (first_coop < levels) {
         F.dsamp = dsamp;
         F.lanes_log2 = pair_lanes_log2(dsamp);
+        F.walk = 0;
         int first = first_coop, nl = levels;
         unsigned* bar = ctx->d_bar;
         unsigned long long limit = (unsigned long long)ctx->barrier_ns;
