@@ -291,7 +291,7 @@ __global__ void k_raygen_multi(const DFrame* __restrict__ T, const int* __restri
 // the n items do not fill 16 warps of an SM each warp takes fewer, down to 4.
 // Thumbnail (128x128 icosphere) 0.387 -> 0.356 ms; the 48 mixed frames of a
 // batch on one lane: trace 33.5 -> 28 ms, cones 67 -> 50 (39 with a thread per
-// light, SPLIT_PAIRS).  With 4 warps of an SM as the limit 29 and 41, with
+// light, SPLIT_HITS).  With 4 warps of an SM as the limit 29 and 41, with
 // 32 no better, and without one the deep levels of large frames lost a third.
 // Spreading frames that do fill the chip costs: the 1080p icosphere 4.49 ms
 // becomes 4.73 with 24 lanes a warp, 5.02 with 16, 5.91 with 8.
@@ -537,10 +537,15 @@ __device__ __forceinline__ bool next_offset(StdRng& rng, double radius, double* 
 // ms; the cones take 0.62, 3.2 and 3.1.  Bound by the latency of its node
 // loads (37% of the issue slots): 8 blocks per SM (64 registers) 3.4 ms on the
 // 1,000-sphere frame where 6 blocks took 3.5 and unbounded (128 registers) 4.0.
-// SPLIT: up to SPLIT_PAIRS pairs of hit and light, each takes a thread of its
-// own.  Frames whose primary rays are far more leave it out: it costs the
-// 1,000-sphere frame 0.3 ms.
-#define SPLIT_PAIRS (1 << 17)
+// SPLIT: up to SPLIT_HITS hits, each pair of hit and light takes a thread of its
+// own, as so few hits leave warps free and a thread's lights queue up: the deep
+// levels of 1,000 spheres under 40 point lights (1280x720) 8.7 -> 5.8 ms, 16
+// lights 3.9 -> 2.8, 12 disk lights 12.4 -> 10.8; with twice the hits 5.6, 2.7,
+// 10.7.  Level 0 of frames whose rays are far more leaves it out, and so do
+// their other levels where a hit has few lights: it costs the 1,000-sphere
+// frame 0.3 ms, and the learned one 0.2 on its deep levels.
+#define SPLIT_HITS (1 << 16)
+
 template <bool COUNT, bool SPLIT>
 __device__ __forceinline__ void shaft_body(const DFrame& F, int level, long long c0, int bid, int nblk,
                                            unsigned* steps = nullptr) {
@@ -552,7 +557,7 @@ __device__ __forceinline__ void shaft_body(const DFrame& F, int level, long long
   Work w{0, 0, 0, 0};
   // one thread per hit, or, where hits are few, per hit and light
   const long long nhc = c1 > c0 ? c1 - c0 : 0;
-  const bool split = SPLIT && S.n_lights > 1 && nhc * S.n_lights <= SPLIT_PAIRS;
+  const bool split = SPLIT && S.n_lights > 1 && nhc <= SPLIT_HITS;
   const long long items = split ? nhc * S.n_lights : nhc;
   const int lanes = walk_lanes(S, items, nblk), wpb = blockDim.x >> 5, lane = threadIdx.x & 31;
   const long long stride = (long long)nblk * wpb * lanes;

@@ -1749,7 +1749,7 @@ rt_status render_impl(rt_ctx* ctx, const rt_scene* sc, const rt_render_params* P
           long long c0 = c * chunk;
           if (c > 0) CK(cudaMemsetAsync(F.pair.n, 0, 8 * sizeof(int), s));  // k_trace cleared them for chunk 0
           const int sgrid = walk_blocks(chunk * std::max(1, n_lights));
-          const bool split = nprim * n_lights <= 32 * SPLIT_PAIRS;
+          const bool split = nprim * n_lights <= 64 * SPLIT_HITS || (l > 0 && n_lights > 4);
           if (count && split) k_shaft<true, true><<<sgrid, 128, 0, s>>>(F, l, c0);
           else if (count) k_shaft<true, false><<<sgrid, 128, 0, s>>>(F, l, c0);
           else if (split) k_shaft<false, true><<<sgrid, 128, 0, s>>>(F, l, c0);
