@@ -940,17 +940,18 @@ __device__ __forceinline__ bool cone_box(const ConeF& f, const float* mn, const 
 // Whether the cone can meet the sphere; *blocks: every ray of the cone is
 // accepted by Sphere::hit (the directions lie inside the sphere's own cone,
 // or o inside the sphere; one root beyond 0.001 and the whole sphere nearer
-// than the disk).
-__device__ __forceinline__ bool cone_sphere(const Cone& k, const double* s, bool* blocks) {
+// than the disk).  endless: the cone goes on beyond the disk.
+__device__ __forceinline__ bool cone_sphere(const Cone& k, const double* s, bool* blocks, bool endless = false) {
   const V3 v = mk(s[0], s[1], s[2]) - k.o;
   const double r = fabs(s[3]);
   const double a = dot(v, k.c), vv = dot(v, v);
-  const double m = 1e-6 * (2.0 * k.D + r);
+  const double end = endless ? fmax(k.D, sum_abs(v) + r) : k.D;  // beyond all of the sphere
+  const double m = 1e-6 * (2.0 * end + r);
   *blocks = false;
   if (!(vv < 1e200)) return true;  // the exact test's discriminant may overflow
-  if (a < -(r + m) || a > k.D + r + m) return false;
+  if (a < -(r + m) || a > end + r + m) return false;
   // apex margin: the point itself may lie on the sphere
-  const double ma = 1e-8 * (k.D + r + sum_abs(k.o)), out2 = (r + ma) * (r + ma);
+  const double ma = 1e-8 * (end + r + sum_abs(k.o)), out2 = (r + ma) * (r + ma);
   if (v.x * k.h[0] + v.y * k.h[1] + v.z * k.h[2] < -(r + ma) * (1.0 + 1e-5)) return false;
   const double p2 = fmax(vv - a * a, 0.0);
   // behind the apex, whose distance then is the cone's: a ca + p sa < 0
@@ -967,23 +968,6 @@ __device__ __forceinline__ bool cone_sphere(const Cone& k, const double* s, bool
     }
   }
   return true;
-}
-
-// Whether the cone can meet the cube, by its bounding sphere.  Cube::hit
-// measures t in the cube's own frame, so a scaled cube may block from beyond
-// the light: its sphere is tested against the cone without an end.
-__device__ __forceinline__ bool cone_cube(const Cone& k, const DCube& C) {
-  const V3 v = ld3(C.bound) - k.o;
-  const double a = dot(v, k.c), vv = dot(v, v);
-  const double r = C.bound[3] * (1.0 + 1e-5) + 1e-5 * sum_abs(v) + 1e-8 * sum_abs(k.o);
-  if (!(vv < 1e200 && r < 1e100) || vv <= r * r) return true;
-  if (C.identity && a > k.D + r) return false;
-  if (v.x * k.h[0] + v.y * k.h[1] + v.z * k.h[2] < -r) return false;
-  const double p2 = fmax(vv - a * a, 0.0);
-  // behind the apex, whose distance then is the cone's
-  if (a < 0.0 && a * a * k.ca * k.ca > p2 * k.sa * k.sa * (1.0 + 1e-5)) return false;
-  const double reach = k.T * a + r / k.ca;
-  return !(reach < 0.0 || p2 > reach * reach);
 }
 
 // Whether the cone can cross the plane through q with normal n (any
@@ -1033,17 +1017,20 @@ __device__ __forceinline__ int shaft_collect(const DScene& S, const Cone& k, int
   for (int i = 0; i < S.n_obj; i++) {
     const int4 ob = __ldg(S.obj + i);
     if (ob.x == OBJ_SPHERE || ob.x == OBJ_PLANE || ob.x == OBJ_CUBE) {
-      bool blocks = false;
-      if (ob.x == OBJ_SPHERE) {
-        if (w) w->spheres++;
-        if (!cone_sphere(k, S.sph + 5 * (size_t)ob.y, &blocks)) continue;
-        if (blocks) return CONE_BLOCKED;
-      } else if (ob.x == OBJ_PLANE) {
+      if (ob.x != OBJ_PLANE) {
+        // a cube by the sphere around it; its own test measures t in its local
+        // frame, so that a scaled cube may block from beyond the light
+        const bool sphere = ob.x == OBJ_SPHERE;
+        bool blocks;
+        if (w && sphere) w->spheres++;
+        if (!cone_sphere(k, sphere ? S.sph + 5 * (size_t)ob.y : S.cub[ob.y].bound, &blocks,
+                         !sphere && !S.cub[ob.y].identity))
+          continue;
+        if (blocks && sphere) return CONE_BLOCKED;
+      } else {
         const double* p = S.pln + 12 * (size_t)ob.y;
         const V3 q = mk(p[0], p[1], p[2]), pn = mk(p[3], p[4], p[5]);
         if (!cone_plane(k, q, pn, sum_abs(pn) * (sum_abs(k.o) + sum_abs(q) + k.D))) continue;
-      } else if (!cone_cube(k, S.cub[ob.y])) {
-        continue;
       }
       if (n == RTB_CAND) return CONE_MANY;
       out[n * stride] = make_int2(i, 0);

@@ -1140,7 +1140,7 @@ void cube_bound(DCube& C, const double a[3][3], const double ai[3][3], bool inve
   }
   const bool box = C.half[0] >= 0.0 && C.half[1] >= 0.0 && C.half[2] >= 0.0;
   for (int k = 0; k < 3; k++) C.bound[k] = C.c[k];
-  C.bound[3] = invertible && box && na * nai < 1e12 && r2 < 1e200 ? std::sqrt(r2) : INFINITY;
+  C.bound[3] = invertible && box && na * nai < 1e12 && r2 < 1e200 ? std::sqrt(r2) * (1.0 + 1e-5) : INFINITY;
 }
 
 rt_status do_upload(rt_ctx* ctx, const rt_scene_desc* d, rt_scene** out,
