@@ -44,14 +44,15 @@ TRAFFIC_FILE = os.path.join(ROOT, "profiles", "k_part_noisy_icosphere_960x540.md
 
 # Algorithmic bytes per unit of work of the shadow kernels (k_shaft, the
 # light cones, and k_part, the sampled lights): every hit's record (68 B) is
-# written once and read once, and each of its lights' results (36 B: state,
-# colour sum, unblocked rays) too, counted here for one light per hit; each
+# written once and read once, and each of its lights' results (32 B: state,
+# colour sum, unblocked rays) too, counted here for one light per hit (an
+# upper bound: of a light that no ray reaches only the state is written); each
 # BVH node visit reads one single-precision node (64 B: two child boxes and
 # their references), each triangle test one triangle record (80 B), each
 # sphere test one sphere (40 B), each verification unit one 16-byte k-d
 # record.  Rays of a light whose cone is empty are not traced and read
 # nothing.
-B_HIT, B_NODE, B_TRI, B_SPH, B_VERIFY = 208, 64, 80, 40, 16
+B_HIT, B_NODE, B_TRI, B_SPH, B_VERIFY = 200, 64, 80, 40, 16
 # FP64 operations per unit (adds, multiplies, divisions and square roots of
 # the restated reference formulas): Moller-Trumbore 40, sphere test 22,
 # verification unit 2.  Node visits test their boxes in single precision

@@ -222,14 +222,15 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 // blockIdx.x, blockIdx.x + gridDim.x, ... (see ConvSeg), a segment's steps
 // down its column, with three roles working on different steps:
 //   warp 4 (TMA): loads input row j (count over the CTA's whole walk) into
-//     ring slot j % NROW with CIN / 8 boxes (8 channels x halo_px pixels of
-//     one row; the hardware zero-fills outside the image and the plane),
-//     once the MMAs of row j - NROW's last step have released the slot;
+//     ring slot j % NROW with one box (all channels x halo_px pixels of one
+//     row, swizzled over the channels' bytes; the hardware zero-fills outside
+//     the image and the plane), once the MMAs of row j - NROW's last step
+//     have released the slot;
 //   warp 5 (MMA): for step t of a segment whose first row is j0, once rows
 //     j0 + t .. j0 + t + 2 have landed and the epilogue has drained
 //     accumulator i % NACC, issues the 9 * CIN / 16 MMAs; tap (ky, kx) reads
 //     row j0 + t + ky's slot from pixel kx * dil on (descriptor start
-//     kx * dil * 16 bytes further); commits to the accumulator's "full"
+//     kx * dil * CIN * 2 bytes further); commits to the accumulator's "full"
 //     barrier and to the "empty" barrier of row j0 + t (and, at a
 //     segment's last step, of its last two rows), each row's last use;
 //   warps 0-3 (epilogue): thread t reads accumulator row t (tcgen05.ld

@@ -158,6 +158,10 @@ __device__ __forceinline__ void tma_row(uint32_t dst, const CUtensorMap* map, in
 // 32 channels: 2.8e-6 of the sum off, 2.5e-8 here (1.4e-7 in FP32 by threads
 // of every 128-pixel run).
 //
+// Beyond a ragged run's end dZ is zero but the shifted inputs are not: an
+// infinite one makes NaN of a tap that does not read it, beside the taps of
+// its channel that do and are not finite either (such a step is skipped).
+//
 // kxs = 1: dilations above 64, whose halo exceeds a TMA box; a step then
 // loads the rows for one kx.
 //
@@ -165,7 +169,7 @@ __device__ __forceinline__ void tma_row(uint32_t dst, const CUtensorMap* map, in
 // and, at few pixels, by the atomics.  It took 3.5 ms of a training step's
 // 4.8 (16 crops of 256x256) when 128 threads transposed every operand tile
 // in registers between two barriers, and takes 0.45 ms now (32 -> 32 channels
-// at full size 56 us; its tensors' bytes take 21).
+// at full size 59 us; its tensors' bytes take 21).
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__ CUtensorMap xmap,
                                                          const __grid_constant__ CUtensorMap zmap, int planes, int H,

@@ -10,6 +10,7 @@
 //   k_part     the disk lights in between: the light's sample points, their
 //              rays and the sum of the unblocked ones' terms, one group of
 //              lanes per (hit, light)
+//   k_walk     k_part's walked pairs, where a level has many
 //   k_light    per hit: ambient + the lights' contributions in the
 //              reference's summation order (unblocked disk lights sampled
 //              here), fog, and the reflection ray, appended to the next
@@ -295,7 +296,8 @@ __global__ void k_raygen_multi(const DFrame* __restrict__ T, const int* __restri
 // 32 no better, and without one the deep levels of large frames lost a third.
 // Spreading frames that do fill the chip costs: the 1080p icosphere 4.49 ms
 // becomes 4.73 with 24 lanes a warp, 5.02 with 16, 5.91 with 8.
-// Scenes without a tree have no walks to spread.
+// Scenes without a tree have no walks to spread.  (16 warps on each of a
+// B200's 148 SMs.)
 #define WALK_WARPS (16 * 148)
 __device__ __forceinline__ int walk_lanes(const DScene& S, long long n, int nblk) {
   const long long warps = min((long long)nblk * (blockDim.x >> 5), (long long)WALK_WARPS);
@@ -531,9 +533,9 @@ __device__ __forceinline__ bool next_offset(StdRng& rng, double radius, double* 
 // Hit records and light classes of hits [c0, c1) of the level's hit list.
 // One thread per hit, one cone per disk light (shaft_collect): where nothing
 // is in the cone, which holds for most hits, the light's rays are never
-// traced.  Lit, listed and walked pairs (with up to eight candidates a
-// list): 1080p icosphere frame 90, 0.2 and 7%, 1,000-sphere frame 69, 15 and
-// 0%, 4K terrain 93, 7 and 0.5%.  Walking every ray took 3.3, 21.5 and 19.1
+// traced.  Lit, listed and walked pairs (counted with up to eight candidates a
+// list and no limit on nodes): 1080p icosphere frame 90, 0.2 and 7%,
+// 1,000-sphere frame 69, 15 and 0%, 4K terrain 93, 7 and 0.5%.  Walking every ray took 3.3, 21.5 and 19.1
 // ms; the cones take 0.62, 3.2 and 3.1.  Bound by the latency of its node
 // loads (37% of the issue slots): 8 blocks per SM (64 registers) 3.4 ms on the
 // 1,000-sphere frame where 6 blocks took 3.5 and unbounded (128 registers) 4.0.
@@ -954,7 +956,7 @@ __device__ __forceinline__ void part_all(const DFrame& F, int level, long long c
 // 1280x720: icosphere under a light as wide as its distance 7.2 -> 6.2 ms, low
 // light over terrain 9.7 -> 8.5, 1,000 spheres under lights of diameter 16 11.0
 // -> 10.2.  Fewer than 2^18 pairs (2^20: the first two as without) fill the
-// chip beside the other queues' blocks, and frames with few walks pay 5 us for
+// chip beside the other queues' blocks, and frames with few walks pay 8 us for
 // a launch that returns.
 template <bool COUNT>
 __global__ void __launch_bounds__(128, 6) k_walk(const __grid_constant__ DFrame F, int level, long long c0) {

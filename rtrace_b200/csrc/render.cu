@@ -241,6 +241,10 @@ const size_t kMaxGraphs = 256;
 
 // The first queue level of k_levels, and the frames it serves: at most this
 // many camera and shadow rays at the primary level, or objects that reflect.
+// The count stands for how much of a frame reflects: a frame with one
+// reflecting plane gains 0.3 of 4.9 ms, one with 1,000 reflecting spheres loses
+// 0.9 of 18.4; in between nothing was measured, and the line lies near the
+// side that keeps the stages' own launches.
 constexpr int kCoopLevel = 2;
 const long long kSmallFrame = 1LL << 22;
 constexpr int kFewReflecting = 4;
